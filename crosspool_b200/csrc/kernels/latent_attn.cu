@@ -120,9 +120,15 @@ latent_prep_kernel(XpLatentPrepArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------ plain kernel
-constexpr int kSimtThreads = 128;
-constexpr int kSimtTile = 32;
-constexpr int kSimtAcc = 8;              // latent columns per thread: kv_rank <= 1024
+//
+// Bound by latency: one head of one row per CTA, a short cache, a dependent chain from page table to row to score to sum. So a
+// tile's page lookups are made together, a warp scores four tokens at a time, and the weighted sum has eight rows in flight
+// (3 decoded rows and portions of 317 in 16 heads over up to 150 tokens of 576: 137 us a launch one row at a time, 46 us so).
+constexpr int kSimtThreads = 256;
+constexpr int kSimtTile = 64;
+constexpr int kSimtAcc = 4;              // latent columns per thread: kv_rank <= 1024
+constexpr int kSimtTokens = 4;           // tokens a warp scores at once
+constexpr int kSimtRows = 8;             // value rows in flight
 
 // First token that a row at the end of len tokens sees.
 __device__ __forceinline__ int window_start(const XpLatentAttnArgs& a, int len) { return a.window > 0 ? max(0, len - a.window) : 0; }
@@ -131,7 +137,8 @@ template <typename T>
 __global__ void __launch_bounds__(kSimtThreads)
 latent_attn_simt_kernel(XpLatentAttnArgs a) {
   extern __shared__ float q_s[];         // kv_rank + rot
-  __shared__ float sc[kSimtTile];
+  __shared__ float sc[kSimtTile], pr[kSimtTile];
+  __shared__ int64_t at[kSimtTile];      // element offsets of the tile's cache rows
   const int h = blockIdx.x, row = blockIdx.y;
   const int dk = a.kv_rank + a.rot;
   T* out = reinterpret_cast<T*>(a.out) + (static_cast<size_t>(h) * a.q_rows + row) * a.ld_out;
@@ -141,45 +148,67 @@ latent_attn_simt_kernel(XpLatentAttnArgs a) {
   }
   const T* q = reinterpret_cast<const T*>(a.q) + (static_cast<size_t>(h) * a.q_rows + row) * a.ld_q;
   for (int c = threadIdx.x; c < dk; c += kSimtThreads) q_s[c] = elem::ld(q + c) * a.scale * kLog2e;
-  __syncthreads();
   const int* table = a.block_table + static_cast<size_t>(a.row_seq != nullptr ? a.row_seq[row] : row) * a.max_blocks;
   const T* cache = reinterpret_cast<const T*>(a.cache);
   const int len = a.positions[row] + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto token_row = [&](int t) {
-    return cache + (static_cast<size_t>(table[t / a.page_size]) * a.page_size + t % a.page_size) * a.ld_cache;
-  };
   float m = -CUDART_INF_F, l = 0.f, acc[kSimtAcc];
 #pragma unroll
   for (int j = 0; j < kSimtAcc; ++j) acc[j] = 0.f;
   for (int t0 = window_start(a, len); t0 < len; t0 += kSimtTile) {
     const int n = min(kSimtTile, len - t0);
-    for (int j = warp; j < n; j += kSimtThreads / 32) {
-      const T* k = token_row(t0 + j);
-      float s = 0.f;
-      for (int c = lane; c < dk; c += 32) s = fmaf(q_s[c], elem::ld(k + c), s);
-      s = elem::warp_sum(s);
-      if (lane == 0) sc[j] = s;
+    __syncthreads();                     // queries are there; the previous tile's rows are consumed
+    if (threadIdx.x < n) {
+      const int t = t0 + threadIdx.x;
+      at[threadIdx.x] = (static_cast<int64_t>(table[t / a.page_size]) * a.page_size + t % a.page_size) * a.ld_cache;
+    }
+    __syncthreads();
+    for (int j0 = warp * kSimtTokens; j0 < n; j0 += kSimtThreads / 32 * kSimtTokens) {
+      const T* k[kSimtTokens];
+      float s[kSimtTokens] = {};
+#pragma unroll
+      for (int i = 0; i < kSimtTokens; ++i) k[i] = cache + at[min(j0 + i, n - 1)];
+#pragma unroll 4
+      for (int c = lane; c < dk; c += 32) {
+        const float qc = q_s[c];
+#pragma unroll
+        for (int i = 0; i < kSimtTokens; ++i) s[i] = fmaf(qc, elem::ld(k[i] + c), s[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < kSimtTokens; ++i) s[i] = elem::warp_sum(s[i]);
+      if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < kSimtTokens; ++i)
+          if (j0 + i < n) sc[j0 + i] = s[i];
+      }
     }
     __syncthreads();
     float mn = m;
     for (int j = 0; j < n; ++j) mn = fmaxf(mn, sc[j]);
+    if (threadIdx.x < kSimtTile) pr[threadIdx.x] = threadIdx.x < n ? exp2f(sc[threadIdx.x] - mn) : 0.f;
     const float f = exp2f(m - mn);       // 0 on the first tile (m = -inf)
     m = mn;
     l *= f;
 #pragma unroll
     for (int j = 0; j < kSimtAcc; ++j) acc[j] *= f;
-    for (int j = 0; j < n; ++j) {
-      const float p = exp2f(sc[j] - m);
-      l += p;
-      const T* v = token_row(t0 + j);
+    __syncthreads();
+    for (int j0 = 0; j0 < n; j0 += kSimtRows) {
+      float v[kSimtRows][kSimtAcc];
 #pragma unroll
-      for (int u = 0; u < kSimtAcc; ++u) {
-        const int c = threadIdx.x + u * kSimtThreads;
-        if (c < a.kv_rank) acc[u] = fmaf(p, elem::ld(v + c), acc[u]);
+      for (int i = 0; i < kSimtRows; ++i)
+#pragma unroll
+        for (int u = 0; u < kSimtAcc; ++u) {
+          const int c = threadIdx.x + u * kSimtThreads;
+          v[i][u] = j0 + i < n && c < a.kv_rank ? elem::ld(cache + at[j0 + i] + c) : 0.f;
+        }
+#pragma unroll
+      for (int i = 0; i < kSimtRows; ++i) {
+        const float p = pr[j0 + i];
+        l += p;
+#pragma unroll
+        for (int u = 0; u < kSimtAcc; ++u) acc[u] = fmaf(p, v[i][u], acc[u]);
       }
     }
-    __syncthreads();
   }
   float g = 1.f / l;
   if (a.gate != nullptr) g *= elem::sigmoid(elem::ld(reinterpret_cast<const T*>(a.gate) + static_cast<size_t>(row) * a.ld_gate + h));
