@@ -61,6 +61,7 @@ typedef struct XpGemmArgs {
   float* tail;
   int ld_tail;
   int relu2;           /* epilogue 0: values are stored as max(value, 0)^2 */
+  int w_static;        /* the kernel before this call on the stream does not write w (model weights): it may be read early */
 } XpGemmArgs;
 
 typedef struct XpGemmPlan {

@@ -104,6 +104,7 @@ struct Problem {
   int tail_from;
   int ld_tail;
   int relu2;               // kEpiStore: features are stored as max(value, 0)^2
+  int w_static;            // weights may be read before the stream's previous kernel has ended
 };
 
 struct SmemLayout {
@@ -241,7 +242,7 @@ __device__ __forceinline__ TileCoord tile_coord(const Problem& p, int t) {
 
 __device__ __forceinline__ bool produce_tile(const Problem& p, const TileCoord& c,
                                              const SmemLayout& L, uint8_t* tiles, Barriers* bar,
-                                             PipeState& st, uint64_t deadline) {
+                                             PipeState& st, uint64_t deadline, int early = 0) {
   const uint64_t pol_w = p.w_evict_first ? sm100::l2_policy_evict_first() : sm100::l2_policy_evict_normal();
   const uint64_t pol_x = sm100::l2_policy_evict_last();
   const uint32_t tx = static_cast<uint32_t>(L.a_bytes + L.b_bytes);
@@ -276,15 +277,17 @@ __device__ __forceinline__ bool produce_tile(const Problem& p, const TileCoord& 
   const bool dual = p.dual != 0;
   for (int i = 0; i < c.kbn; ++i) {
     const uint32_t full = full0 + stage * 8, empty = empty0 + stage * 8;
-    if (!sm100::mbar_try_wait_addr(empty, phase ^ 1) &&
-        !sm100::mbar_wait_addr(empty, phase ^ 1, deadline)) {
-      st.stage = stage;
-      st.phase = phase;
-      return false;
+    if (i >= early) {
+      if (!sm100::mbar_try_wait_addr(empty, phase ^ 1) &&
+          !sm100::mbar_wait_addr(empty, phase ^ 1, deadline)) {
+        st.stage = stage;
+        st.phase = phase;
+        return false;
+      }
+      sm100::mbar_arrive_expect_tx_addr(full, tx);
+      sm100::tma_load_2d_addr(a_addr, tw, full, wc0, wc1, pol_w);
+      if (dual) sm100::tma_load_2d_addr(a_addr + kTileM * kTileK * 2, tw, full, wc0, uc1, pol_w);
     }
-    sm100::mbar_arrive_expect_tx_addr(full, tx);
-    sm100::tma_load_2d_addr(a_addr, tw, full, wc0, wc1, pol_w);
-    if (dual) sm100::tma_load_2d_addr(a_addr + kTileM * kTileK * 2, tw, full, wc0, uc1, pol_w);
     sm100::tma_load_2d_addr(a_addr + a_bytes, tx_map, full, xc0, c.n0, pol_x);
     wc0 += dwc0;
     wc1 += dwc1;
@@ -300,6 +303,24 @@ __device__ __forceinline__ bool produce_tile(const Problem& p, const TileCoord& 
   st.stage = stage;
   st.phase = phase;
   return true;
+}
+
+// Requests the weights of the first K blocks of a CTA's first tile (as many as there are stages) before the activations
+// are there; produce_tile is told how many and requests only the activations of those.
+__device__ __forceinline__ int preload_weights(const Problem& p, const TileCoord& c, const SmemLayout& L, uint8_t* tiles, Barriers* bar) {
+  const uint64_t pol_w = p.w_evict_first ? sm100::l2_policy_evict_first() : sm100::l2_policy_evict_normal();
+  const uint64_t tw = reinterpret_cast<uint64_t>(p.tmap_w);
+  const uint32_t tiles_addr = sm100::smem_u32(tiles);
+  const int n = c.kbn < L.stages ? c.kbn : L.stages, kb_total = k_blocks(p);
+  for (int i = 0; i < n; ++i) {
+    const uint32_t full = sm100::smem_u32(&bar->full[i]), dst = tiles_addr + i * L.stage_bytes;
+    const int col = p.w_tiled ? 0 : (c.kb0 + i) * p.kblk;
+    auto row = [&](int r) { return p.w_tiled ? ((r / kTileM) * kb_total + c.kb0 + i) * kTileM : r; };
+    sm100::mbar_arrive_expect_tx_addr(full, static_cast<uint32_t>(L.a_bytes + L.b_bytes));
+    sm100::tma_load_2d_addr(dst, tw, full, col, row(c.w_row0), pol_w);
+    if (p.dual) sm100::tma_load_2d_addr(dst + kTileM * kTileK * 2, tw, full, col, row(p.up_offset + c.w_row0), pol_w);
+  }
+  return n;
 }
 
 // After a failed wait: give loads still in flight a bounded time to land so that

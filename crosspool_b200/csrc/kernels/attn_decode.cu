@@ -14,6 +14,7 @@
 #include "xpool/api.h"
 #include "xpool/sm100.cuh"
 #include "xpool/tensormap.hpp"
+#include "xpool/pdl.cuh"
 
 namespace xpool {
 namespace attn {
@@ -378,6 +379,8 @@ template <int DQ, int DV, typename A, bool kSig = false>
 __global__ void __launch_bounds__(kDecodeThreads, 2)
 decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                       const __grid_constant__ CUtensorMap tmap_kp, const __grid_constant__ CUtensorMap tmap_vp, A args) {
+  pdl::wait();
+  pdl::release();
   constexpr bool kRows = std::is_same<A, XpDecodeRowsArgs>::value;
   static_assert(kRows || !kSig, "sigmoid weights are a form of single rows");
   const XpDecodeAttnArgs& a = base_of(args);
@@ -707,6 +710,8 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 
 template <int D, bool kSig = false, typename A>
 __global__ void decode_combine_kernel(A args, int nsplit) {
+  pdl::wait();
+  pdl::release();
   const XpDecodeAttnArgs& a = base_of(args);
   const int hq = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const float* ws = a.ws + (static_cast<size_t>(b) * a.q_heads + hq) * nsplit * (D + 2);
@@ -736,7 +741,7 @@ static int launch_decode(const XpDecodeAttnArgs& a, int nsplit, cudaStream_t s) 
     attr_set = true;
   }
   decode_attn_kernel<D, GMAX><<<grid, kDecodeThreads, kRing, s>>>(a);
-  if (nsplit > 1) decode_combine_kernel<D><<<dim3(a.q_heads, a.batch), D, 0, s>>>(a, nsplit);
+  if (nsplit > 1) pdl::launch(decode_combine_kernel<D, false, XpDecodeAttnArgs>, dim3(a.q_heads, a.batch), D, 0, s, 1, a, nsplit);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }
@@ -765,8 +770,8 @@ static int launch_decode_tc(const A& args, int nsplit, cudaStream_t s) {
     attr_set = true;
   }
   dim3 grid(nsplit, a.kv_heads, a.batch);
-  decode_attn_tc_kernel<DQ, DV, A, kSig><<<grid, kDecodeThreads, kSmem, s>>>(mk, mv, mkp, mvp, args);
-  if (nsplit > 1) decode_combine_kernel<DV, kSig><<<dim3(a.q_heads, a.batch), DV, 0, s>>>(args, nsplit);
+  pdl::launch(decode_attn_tc_kernel<DQ, DV, A, kSig>, grid, kDecodeThreads, kSmem, s, 1, mk, mv, mkp, mvp, args);
+  if (nsplit > 1) pdl::launch(decode_combine_kernel<DV, kSig, A>, dim3(a.q_heads, a.batch), DV, 0, s, 1, args, nsplit);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }

@@ -41,6 +41,7 @@
 #include "xpool/api.h"
 #include "xpool/sm100.cuh"
 #include "xpool/tensormap.hpp"
+#include "xpool/pdl.cuh"
 
 namespace xpool {
 namespace attn5 {
@@ -168,6 +169,7 @@ prefill_attn_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   __shared__ Bars bars;
 
   const int np = kRows >> g_shift;                // query positions per tile
+  pdl::wait();
   // blocks are dispatched x-fastest: (head, sequence) vary fastest and the query tile slowest, so that the tiles with
   // the longest key range of every head and sequence start first and the short ones fill the tail
   const int hk = blockIdx.x, seq = blockIdx.y, qt = static_cast<int>(gridDim.z) - 1 - static_cast<int>(blockIdx.z);
@@ -224,6 +226,7 @@ prefill_attn_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   __syncthreads();
   sm100::tc_fence_after_sync();
   const uint32_t tmem = bars.tmem_base;
+  pdl::release();
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
@@ -638,7 +641,7 @@ static int launch(const XpPrefillAttnArgs& a, int G, cudaStream_t s) {
   if (b.ld_out <= 0) b.ld_out = b.q_heads * b.v_valid;
   if (b.group_valid <= 0) b.group_valid = G;
   dim3 grid(b.kv_heads, b.num_seqs, (b.max_q_len + 2 * np - 1) / (2 * np));
-  prefill_attn_umma_kernel<DQ, DV, kTS, kPair, kCap, kSig><<<grid, kThreads, kSmem, s>>>(mq, mk, mv, mk3, mv3, mkp, mvp, b, G, g_shift, box_tokens);
+  pdl::launch(prefill_attn_umma_kernel<DQ, DV, kTS, kPair, kCap, kSig>, grid, kThreads, kSmem, s, 1, mq, mk, mv, mk3, mv3, mkp, mvp, b, G, g_shift, box_tokens);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }

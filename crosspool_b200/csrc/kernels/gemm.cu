@@ -3,8 +3,10 @@
 #include <algorithm>
 
 #include "xpool/api.h"
+#include "xpool/gemm_stream.cuh"
 #include "xpool/gemm_ws.cuh"
 #include "xpool/lane.cuh"
+#include "xpool/pdl.cuh"
 #include "xpool/tensormap.hpp"
 
 namespace xpool {
@@ -21,16 +23,25 @@ __device__ __forceinline__ void run_tiles(const Problem& p, int nacc, int smem_b
   const uint32_t tmem_cols = tmem_columns_needed(p.bn, p.dual, nacc);
   Barriers* bar;
   uint8_t* tiles = cta_setup(smem_raw, L, &bar, tmem_cols, warp, lane);
+  // Set-up and the first weight tiles do not depend on the stream's previous kernel; everything below does (the Lane form is
+  // an ordinary launch, where the wait returns at once).
+  int early = 0;
+  if (warp == 0 && lane == 0) {
+    sm100::tma_prefetch_desc(p.tmap_w);
+    sm100::tma_prefetch_desc(p.tmap_x);
+    if (p.w_static && p.tile_table == nullptr && static_cast<int>(blockIdx.x) < tile_count(p))
+      early = preload_weights(p, tile_coord(p, blockIdx.x), L, tiles, bar);
+  }
+  pdl::wait();
+  pdl::release();
   const int ntiles = tile_count(p);
 
   if (warp == 0) {
     if (lane == 0) {
-      sm100::tma_prefetch_desc(p.tmap_w);
-      sm100::tma_prefetch_desc(p.tmap_x);
       PipeState st;
       for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const uint64_t deadline = sm100::global_timer_ns() + sm100::kPipelineWaitNs;
-        if (!produce_tile(p, tile_coord(p, t), L, tiles, bar, st, deadline)) {
+        if (!produce_tile(p, tile_coord(p, t), L, tiles, bar, st, deadline, t == static_cast<int>(blockIdx.x) ? early : 0)) {
           record_status(status, kTimeoutProducer);
           producer_drain(L, bar, st);
           break;
@@ -336,6 +347,7 @@ extern "C" int xp_gemm(const XpGemmArgs* a) {
   XpGemmPlan plan;
   int rc = xp_gemm_plan(a, &plan);
   if (rc != 0) return rc;
+  if (gemm::stream_applies(*a)) return gemm::stream_launch(*a);
   if (plan.splits > 1) {
     if (a->ws == nullptr || a->counters == nullptr || a->ws_bytes < plan.ws_bytes ||
         a->counter_bytes < plan.counter_bytes) {
@@ -405,6 +417,7 @@ extern "C" int xp_gemm(const XpGemmArgs* a) {
   p.tail_from = a->tail_from;
   p.ld_tail = a->ld_tail;
   p.relu2 = a->relu2;
+  p.w_static = a->w_static;
   if (a->tile_table != nullptr) {
     if (plan.splits != 1) return -13;
     plan.grid = plan.smem_bytes > 0 ? 148 : 148;
@@ -425,7 +438,7 @@ extern "C" int xp_gemm(const XpGemmArgs* a) {
   }
   const bool wide = p.act_cubic != 0.f || p.epilogue == gemm::kEpiGateMul || p.epilogue == gemm::kEpiSigmoid || p.tail != nullptr || p.relu2 != 0;
   auto kernel = wide ? gemm::gemm_ws_kernel<true> : gemm::gemm_ws_kernel<false>;
-  kernel<<<plan.grid, gemm::kThreads, plan.smem_bytes, reinterpret_cast<cudaStream_t>(a->stream)>>>(tw, tx, p, plan.nacc, plan.smem_budget, a->status);
+  pdl::launch(kernel, plan.grid, gemm::kThreads, plan.smem_bytes, reinterpret_cast<cudaStream_t>(a->stream), 1, tw, tx, p, plan.nacc, plan.smem_budget, a->status);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }

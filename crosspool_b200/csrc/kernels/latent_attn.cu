@@ -17,6 +17,7 @@
 #include "xpool/elem.cuh"
 #include "xpool/mixer_api.h"
 #include "xpool/sm100.cuh"
+#include "xpool/pdl.cuh"
 
 namespace xpool {
 namespace latent {
@@ -30,6 +31,8 @@ constexpr int kPrepHeads = 8;              // heads per CTA (grid y): one per wa
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kPrepThreads)
 latent_prep_kernel(XpLatentPrepArgs a) {
+  pdl::wait();
+  pdl::release();
   extern __shared__ float cs[];            // cos | sin, rot_dims / 2 each
   __shared__ float red[kPrepThreads / 32];
   const int row = blockIdx.x;
@@ -136,6 +139,8 @@ __device__ __forceinline__ int window_start(const XpLatentAttnArgs& a, int len) 
 template <typename T>
 __global__ void __launch_bounds__(kSimtThreads)
 latent_attn_simt_kernel(XpLatentAttnArgs a) {
+  pdl::wait();
+  pdl::release();
   extern __shared__ float q_s[];         // kv_rank + rot
   __shared__ float sc[kSimtTile], pr[kSimtTile];
   __shared__ int64_t at[kSimtTile];      // element offsets of the tile's cache rows
@@ -300,6 +305,8 @@ __device__ __forceinline__ bool compute_any(bool p) {
 template <int NT, int HG>
 __global__ void __launch_bounds__(kTcThreads)
 latent_attn_tc_kernel(XpLatentAttnArgs a) {
+  pdl::wait();
+  pdl::release();
   extern __shared__ __align__(16) uint8_t smem[];
   constexpr int MH = 16 * HG;                        // heads of the CTA
   const int split = blockIdx.x, h0 = blockIdx.y * MH, row = blockIdx.z;
@@ -568,6 +575,8 @@ constexpr int kMaxSlices = 64;
 // One CTA per (head, row): folds the slices in order.
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(XpLatentAttnArgs a) {
+  pdl::wait();
+  pdl::release();
   const int h = blockIdx.x, row = blockIdx.y;
   const bool pad = a.slots[row] < 0;
   const int len = pad ? 0 : a.positions[row] + 1;
@@ -649,8 +658,8 @@ int launch_tc(const XpLatentAttnArgs& a, cudaStream_t s) {
     set = true;
   }
   dim3 grid(a.num_splits > 1 ? a.num_splits : 1, (a.heads + 16 * HG - 1) / (16 * HG), a.rows);
-  latent_attn_tc_kernel<NT, HG><<<grid, kTcThreads, L.total, s>>>(a);
-  if (a.num_splits > 1) latent_merge_kernel<<<dim3(a.heads, a.rows), 128, 0, s>>>(a);
+  xpool::pdl::launch(latent_attn_tc_kernel<NT, HG>, grid, kTcThreads, L.total, s, 1, a);
+  if (a.num_splits > 1) xpool::pdl::launch(latent_merge_kernel, dim3(a.heads, a.rows), 128, 0, s, 1, a);
   return done();
 }
 
@@ -676,11 +685,11 @@ extern "C" int xp_latent_prep(const XpLatentPrepArgs* a, void* stream) {
                  al(a->proj) && al(a->q_plain) && al(a->q_exp) && al(a->q) && a->ld_q % 4 == 0 && a->q_rank % 4 == 0 && a->ql_off % 4 == 0;
   dim3 grid(a->rows, (a->heads + kPrepHeads - 1) / kPrepHeads);
   if (a->f32) {
-    if (v) latent_prep_kernel<float, 4><<<grid, kPrepThreads, sm, s>>>(*a);
-    else latent_prep_kernel<float, 1><<<grid, kPrepThreads, sm, s>>>(*a);
+    if (v) xpool::pdl::launch(latent_prep_kernel<float, 4>, grid, kPrepThreads, sm, s, 1, *a);
+    else xpool::pdl::launch(latent_prep_kernel<float, 1>, grid, kPrepThreads, sm, s, 1, *a);
   } else {
-    if (v) latent_prep_kernel<__nv_bfloat16, 4><<<grid, kPrepThreads, sm, s>>>(*a);
-    else latent_prep_kernel<__nv_bfloat16, 1><<<grid, kPrepThreads, sm, s>>>(*a);
+    if (v) xpool::pdl::launch(latent_prep_kernel<__nv_bfloat16, 4>, grid, kPrepThreads, sm, s, 1, *a);
+    else xpool::pdl::launch(latent_prep_kernel<__nv_bfloat16, 1>, grid, kPrepThreads, sm, s, 1, *a);
   }
   return done();
 }
@@ -699,8 +708,8 @@ extern "C" int xp_latent_attn(const XpLatentAttnArgs* a, void* stream) {
   if (a->kv_rank > kSimtAcc * kSimtThreads || a->kv_rank + a->rot > 12000) return -12;
   dim3 grid(a->heads, a->rows);
   const size_t sm = static_cast<size_t>(a->kv_rank + a->rot) * 4;
-  if (a->f32) latent_attn_simt_kernel<float><<<grid, kSimtThreads, sm, s>>>(*a);
-  else latent_attn_simt_kernel<__nv_bfloat16><<<grid, kSimtThreads, sm, s>>>(*a);
+  if (a->f32) xpool::pdl::launch(latent_attn_simt_kernel<float>, grid, kSimtThreads, sm, s, 1, *a);
+  else xpool::pdl::launch(latent_attn_simt_kernel<__nv_bfloat16>, grid, kSimtThreads, sm, s, 1, *a);
   return done();
 }
 

@@ -8,6 +8,7 @@
 #include "xpool/mixer_api.h"
 #include "xpool/mma_sync.cuh"
 #include "xpool/sm100.cuh"
+#include "xpool/pdl.cuh"
 
 namespace xpool {
 namespace linear {
@@ -19,6 +20,8 @@ constexpr int kThreads = 256;
 template <typename T, int N>
 __global__ void __launch_bounds__(kThreads)
 linear_decode_kernel(XpLinearAttnArgs a) {
+  pdl::wait();
+  pdl::release();
   extern __shared__ float sm[];            // q[dim], k[dim], partial sums [groups][vdim]
   const int h = blockIdx.x, row = blockIdx.y;
   float* out = a.out + static_cast<size_t>(row) * a.heads * a.vdim + static_cast<size_t>(h) * a.vdim;
@@ -487,7 +490,7 @@ int launch_decode(const XpLinearAttnArgs& a, cudaStream_t s) {
   const size_t sm = static_cast<size_t>(2 * a.dim + groups * a.vdim) * 4;
   int rc = big_smem(linear_decode_kernel<T, N>, sm);
   if (rc != 0) return rc;
-  linear_decode_kernel<T, N><<<dim3(a.heads, a.rows), kThreads, sm, s>>>(a);
+  xpool::pdl::launch(linear_decode_kernel<T, N>, dim3(a.heads, a.rows), kThreads, sm, s, 1, a);
   return done();
 }
 

@@ -12,6 +12,7 @@
 // by a system-scope release of a sequence word.
 #include "xpool/api.h"
 #include "xpool/hooks.cuh"
+#include "xpool/pdl.cuh"
 #include "xpool/sm100.cuh"
 
 namespace xpool {
@@ -45,6 +46,9 @@ constexpr int kMaxVec = 4;  // 256 threads * 8 elems * 4 = 8192 hidden max
 
 __global__ void __launch_bounds__(kThreads)
 norm_publish_kernel(XpNormArgs a) {
+  // A CTA that may spin on another GPU's flag holds its successor back: CTAs resident early would take the room of what it waits for.
+  pdl::wait();
+  if (a.wait_seq == 0 && a.npeers == 0) pdl::release();
   __shared__ float red[kThreads / 32];
   __shared__ uint32_t s_fail;
   const int row = blockIdx.x;
@@ -206,8 +210,7 @@ swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ 
 extern "C" int xp_norm_publish(const XpNormArgs* a, void* stream) {
   if (a->hidden % 8 != 0 || a->hidden > 8 * xpool::norm::kThreads * xpool::norm::kMaxVec) return -10;
   if (a->rows <= 0 || a->nparts < 1 || a->nparts > 8 || a->npeers < 0 || a->npeers > 8) return -11;
-  xpool::norm::norm_publish_kernel<<<a->rows, xpool::norm::kThreads, 0,
-                                     reinterpret_cast<cudaStream_t>(stream)>>>(*a);
+  xpool::pdl::launch(xpool::norm::norm_publish_kernel, a->rows, xpool::norm::kThreads, 0, reinterpret_cast<cudaStream_t>(stream), 1, *a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }

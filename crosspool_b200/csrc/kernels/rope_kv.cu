@@ -8,6 +8,7 @@
 // for V; `slots[row]` = page * page_size + offset, or -1 for padding rows.
 #include "xpool/api.h"
 #include "xpool/sm100.cuh"
+#include "xpool/pdl.cuh"
 
 namespace xpool {
 namespace rope {
@@ -15,6 +16,8 @@ namespace rope {
 template <int D>
 __global__ void __launch_bounds__(256)
 rope_kv_kernel(XpRopeArgs a) {
+  pdl::wait();
+  pdl::release();
   constexpr int PER = D / 64;  // elements per lane in each half
   const int row = blockIdx.x;
   const int head = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -89,9 +92,9 @@ extern "C" int xp_rope_kv(const XpRopeArgs* a, void* stream) {
   dim3 grid(a->rows, (heads_total + 7) / 8);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (a->head_dim == 128)
-    xpool::rope::rope_kv_kernel<128><<<grid, 256, 0, s>>>(*a);
+    xpool::pdl::launch(xpool::rope::rope_kv_kernel<128>, grid, 256, 0, s, 1, *a);
   else if (a->head_dim == 64)
-    xpool::rope::rope_kv_kernel<64><<<grid, 256, 0, s>>>(*a);
+    xpool::pdl::launch(xpool::rope::rope_kv_kernel<64>, grid, 256, 0, s, 1, *a);
   else
     return -10;
   cudaError_t e = cudaGetLastError();

@@ -9,6 +9,7 @@
 // Rows whose pitches allow it are moved four elements at a time.
 #include "xpool/elem.cuh"
 #include "xpool/mixer_api.h"
+#include "xpool/pdl.cuh"
 
 namespace xpool {
 namespace rowops {
@@ -24,6 +25,8 @@ enum NormKind : int { kRms = 0, kLayer = 1, kDynTanh = 2 };
 template <typename T, int N, int KIND>
 __global__ void __launch_bounds__(kThreads)
 resid_norm_kernel(XpResidNormArgs a) {
+  pdl::wait();
+  pdl::release();
   __shared__ float red[kThreads / 32];
   const int i = blockIdx.x;
   const int r = a.sel != nullptr ? a.sel[i] : i;
@@ -120,6 +123,8 @@ constexpr int kKeep = 32;
 template <typename T, int N>
 __global__ void __launch_bounds__(kThreads)
 polynorm_kernel(XpPolyNormArgs a) {
+  pdl::wait();
+  pdl::release();
   __shared__ float red[kThreads / 32];
   const T* z = reinterpret_cast<const T*>(a.z) + static_cast<size_t>(blockIdx.x) * a.ld_z;
   T* out = reinterpret_cast<T*>(a.out) + static_cast<size_t>(blockIdx.x) * a.ld_out;
@@ -171,6 +176,8 @@ polynorm_kernel(XpPolyNormArgs a) {
 template <typename T, int N>
 __global__ void __launch_bounds__(kThreads)
 gated_rms_kernel(XpGatedRmsArgs a) {
+  pdl::wait();
+  pdl::release();
   __shared__ float red[kThreads / 32];
   const float* o = a.o + static_cast<size_t>(blockIdx.x) * a.ld_o;
   const T* gate = reinterpret_cast<const T*>(a.gate) + static_cast<size_t>(blockIdx.x) * a.ld_gate;
@@ -348,9 +355,9 @@ inline bool vec4(const void* p, int64_t ld, int elem_bytes) {
 
 template <typename T, int N>
 void launch_resid(const XpResidNormArgs& a, cudaStream_t s) {
-  if (a.kind == kRms) resid_norm_kernel<T, N, kRms><<<a.rows, kThreads, 0, s>>>(a);
-  else if (a.kind == kLayer) resid_norm_kernel<T, N, kLayer><<<a.rows, kThreads, 0, s>>>(a);
-  else resid_norm_kernel<T, N, kDynTanh><<<a.rows, kThreads, 0, s>>>(a);
+  if (a.kind == kRms) xpool::pdl::launch(resid_norm_kernel<T, N, kRms>, a.rows, kThreads, 0, s, 1, a);
+  else if (a.kind == kLayer) xpool::pdl::launch(resid_norm_kernel<T, N, kLayer>, a.rows, kThreads, 0, s, 1, a);
+  else xpool::pdl::launch(resid_norm_kernel<T, N, kDynTanh>, a.rows, kThreads, 0, s, 1, a);
 }
 
 template <typename T, int N>
@@ -393,11 +400,11 @@ extern "C" int xp_polynorm(const XpPolyNormArgs* a, void* stream) {
   const bool v = a->cols % 4 == 0 && vec4(a->z, a->ld_z, eb) && vec4(a->out, a->ld_out, eb);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (a->f32) {
-    if (v) polynorm_kernel<float, 4><<<a->rows, kThreads, 0, s>>>(*a);
-    else polynorm_kernel<float, 1><<<a->rows, kThreads, 0, s>>>(*a);
+    if (v) xpool::pdl::launch(polynorm_kernel<float, 4>, a->rows, kThreads, 0, s, 1, *a);
+    else xpool::pdl::launch(polynorm_kernel<float, 1>, a->rows, kThreads, 0, s, 1, *a);
   } else {
-    if (v) polynorm_kernel<__nv_bfloat16, 4><<<a->rows, kThreads, 0, s>>>(*a);
-    else polynorm_kernel<__nv_bfloat16, 1><<<a->rows, kThreads, 0, s>>>(*a);
+    if (v) xpool::pdl::launch(polynorm_kernel<__nv_bfloat16, 4>, a->rows, kThreads, 0, s, 1, *a);
+    else xpool::pdl::launch(polynorm_kernel<__nv_bfloat16, 1>, a->rows, kThreads, 0, s, 1, *a);
   }
   return done();
 }
@@ -410,11 +417,11 @@ extern "C" int xp_gated_rms(const XpGatedRmsArgs* a, void* stream) {
                  vec4(a->out, a->ld_out, eb);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (a->f32) {
-    if (v) gated_rms_kernel<float, 4><<<a->rows, kThreads, 0, s>>>(*a);
-    else gated_rms_kernel<float, 1><<<a->rows, kThreads, 0, s>>>(*a);
+    if (v) xpool::pdl::launch(gated_rms_kernel<float, 4>, a->rows, kThreads, 0, s, 1, *a);
+    else xpool::pdl::launch(gated_rms_kernel<float, 1>, a->rows, kThreads, 0, s, 1, *a);
   } else {
-    if (v) gated_rms_kernel<__nv_bfloat16, 4><<<a->rows, kThreads, 0, s>>>(*a);
-    else gated_rms_kernel<__nv_bfloat16, 1><<<a->rows, kThreads, 0, s>>>(*a);
+    if (v) xpool::pdl::launch(gated_rms_kernel<__nv_bfloat16, 4>, a->rows, kThreads, 0, s, 1, *a);
+    else xpool::pdl::launch(gated_rms_kernel<__nv_bfloat16, 1>, a->rows, kThreads, 0, s, 1, *a);
   }
   return done();
 }

@@ -351,15 +351,15 @@ class AttentionEngine:
             else:
                 norm.add_rmsnorm(weight=lw.input_norm, eps=cfg.rms_norm_eps, resid=resid, out=x, **_parts_kw(parts),
                                  **self.port.wait_args())
-            gemm.linear(x, lw.qkv, out=self.qkv[:rows], bias=lw.qkv_bias)
+            gemm.linear(x, lw.qkv, out=self.qkv[:rows], bias=lw.qkv_bias, w_static=True)
             attn_fn(l, lw, rows)
             tgt = self.port.publish_targets(l, rows, mode)
             if self.tp is None:
-                gemm.linear(self.attn_out[:rows].view(rows, cfg.q_size), lw.o, out=self.o[:rows])
+                gemm.linear(self.attn_out[:rows].view(rows, cfg.q_size), lw.o, out=self.o[:rows], w_static=True)
                 o_parts = dict(parts=[self.o[:rows]])
             else:
                 # this rank's heads give a partial; all ranks' partials are folded by the norm below
-                gemm.linear(self.attn_out[:rows].view(rows, cfg.q_size), lw.o, out=self.tp.part(l)[:rows])
+                gemm.linear(self.attn_out[:rows].view(rows, cfg.q_size), lw.o, out=self.tp.part(l)[:rows], w_static=True)
                 self.tp.exchange()
                 o_parts = dict(parts=[], part_ptrs=self.tp.part_ptrs(l), part_shape=(rows, cfg.hidden_size, cfg.hidden_size))
             if tgt is None:
@@ -380,7 +380,7 @@ class AttentionEngine:
             hsel = self.x[:n_sel]
         else:
             hsel = A.embedding(sel_idx, self.x[:rows], out=self.sel[:n_sel])
-        gemm.linear(hsel, self.w.lm_head, out=self.logits[:n_sel])
+        gemm.linear(hsel, self.w.lm_head, out=self.logits[:n_sel], w_static=True)
         self._sample(n_sel)
 
     def _sample(self, n_sel: int) -> None:

@@ -61,10 +61,10 @@ class LocalFfnPort(FfnPort):
 
         ff = w.gate_up.shape[0]
         z = self.act[:rows * ceil8(ff)].view(rows, ceil8(ff))[:, :ff]
-        gemm.linear(x, w.gate_up, out=z)
+        gemm.linear(x, w.gate_up, out=z, w_static=True)
         coef, eps = w.extra["polynorm"]
         mixers.polynorm(z, coef, eps, z)
-        gemm.linear(z, w.down, out=self.y[:rows])
+        gemm.linear(z, w.down, out=self.y[:rows], w_static=True)
         return [self.y[:rows]]
 
     def _run_gated(self, w: FfnLayerWeights, x: torch.Tensor, rows: int) -> list[torch.Tensor]:
@@ -76,11 +76,11 @@ class LocalFfnPort(FfnPort):
             from ..ops import mixers
 
             z = self.act[rows * ceil8(ff):][:rows * 2 * ff].view(rows, 2 * ff)
-            gemm.linear(x, w.gate_up, out=z)
+            gemm.linear(x, w.gate_up, out=z, w_static=True)
             mixers.glu_f32(z, limit, up_add, alpha, act, cubic)
         else:
-            gemm.gateup_swiglu(x, w.gate_up, out=act, gate_limit=limit, up_add=up_add, act_alpha=alpha, act_cubic=cubic)
-        gemm.linear(act, w.down, out=self.y[:rows])
+            gemm.gateup_swiglu(x, w.gate_up, out=act, gate_limit=limit, up_add=up_add, act_alpha=alpha, act_cubic=cubic, w_static=True)
+        gemm.linear(act, w.down, out=self.y[:rows], w_static=True)
         return [self.y[:rows]]
 
     def run(self, layer: int, x: torch.Tensor, rows: int, mode: int) -> list[torch.Tensor]:
@@ -102,8 +102,8 @@ class LocalFfnPort(FfnPort):
         inter = w.gate_up.shape[0] // 2
         act = self.act[:rows, :inter]
         lim, up_add, alpha = w.extra.get("gate_transform", (0.0, 0.0, 0.0))
-        gemm.gateup_swiglu(x, w.gate_up, out=act, bias=w.gate_up_bias, gate_limit=lim, up_add=up_add, act_alpha=alpha)
-        gemm.linear(act, w.down, out=self.y[:rows], bias=w.down_bias)
+        gemm.gateup_swiglu(x, w.gate_up, out=act, bias=w.gate_up_bias, gate_limit=lim, up_add=up_add, act_alpha=alpha, w_static=True)
+        gemm.linear(act, w.down, out=self.y[:rows], bias=w.down_bias, w_static=True)
         return [self.y[:rows]]
 
 

@@ -169,12 +169,12 @@ class LayeredForward:
         if m.q_rank:
             n = m.heads * (m.dim + m.rot_dim)
             q = self.q_lat[:rows * ceil8(n)].view(rows, ceil8(n))[:, :n]
-            gemm.linear(proj[:, q_off:q_off + m.q_rank], lw.mix["uq"], out=q)
+            gemm.linear(proj[:, q_off:q_off + m.q_rank], lw.mix["uq"], out=q, w_static=True)
         M.latent_prep(proj, lw.mix["norm"], lw.mix["freq"], b.positions, b.slots, cache, heads=H, dim=m.dim, rot=m.rot_dim, kv_rank=R,
                       q_off=q_off, kv_off=lw.offs["kv"], eps=self.e.cfg.rms_norm_eps, abs_rows=n_abs, q_plain=q_plain,
                       q_abs=q_abs, q_exp=q_exp, q=q, q_rank=m.q_rank, interleaved=m.rot.interleaved)
         if n_abs:
-            gemm.linear_batched(q_plain[:, :, :m.dim], lw.mix["uk_t"], q_abs, n_abs * W)
+            gemm.linear_batched(q_plain[:, :, :m.dim], lw.mix["uk_t"], q_abs, n_abs * W, w_static=True)
             splits, chunk = M.latent_attn_plan(n_abs, H, m.visible(b.max_len), W)
             if splits > 1 and n_abs * H * splits * (R + 2) > self.attn_ws.numel():
                 splits, chunk = 1, 0
@@ -182,7 +182,7 @@ class LayeredForward:
             M.latent_attn(q_abs, cache, o_lat, b.table, b.positions, b.slots, kv_rank=R, rot=m.rot_dim, scale=m.scale,
                           gate=None if m.gate_elems else gate, row_seq=b.row_seq, num_splits=splits, chunk_tokens=chunk, ws=self.attn_ws,
                           window=m.window)
-            gemm.linear_batched(o_lat[:, :, :R], lw.mix["uv"], out[:n_abs], m.vdim, gate=gate[:n_abs] if m.gate_elems else None)
+            gemm.linear_batched(o_lat[:, :, :R], lw.mix["uv"], out[:n_abs], m.vdim, gate=gate[:n_abs] if m.gate_elems else None, w_static=True)
         if n_abs < rows:
             for g in b.groups:
                 s = slice(g.seq0, g.seq0 + g.n)
@@ -191,8 +191,8 @@ class LayeredForward:
                 M.latent_gather(cache, lat, b.table[s], b.ctx_lens[s], b.q_lens[s], starts, g.max_len, m.window)
                 k = self.k_exp[:g.tokens * H * dq].view(g.tokens, H, dq)
                 v = self.v_exp[:g.tokens * H * dv].view(g.tokens, H, dv)
-                gemm.linear(lat[:, :R + m.rot_dim], lw.mix["exp_k"], out=k.view(g.tokens, H * dq))
-                gemm.linear(lat[:, :R], lw.mix["exp_v"], out=v.view(g.tokens, H * dv))
+                gemm.linear(lat[:, :R + m.rot_dim], lw.mix["exp_k"], out=k.view(g.tokens, H * dq), w_static=True)
+                gemm.linear(lat[:, :R], lw.mix["exp_v"], out=v.view(g.tokens, H * dv), w_static=True)
                 M.expanded_prefill(q_exp, k, v, out, b.q_starts[s], b.q_lens[s], b.ctx_lens[s], starts, g.max_q, scale=m.scale,
                                    vdim=m.vdim, gate=gate, window=m.window)
 
@@ -294,7 +294,7 @@ class LayeredForward:
         if nd < b.n_seqs:
             s = slice(nd, b.n_seqs)
             z = self.z[:b.rows * m.heads * m.dim].view(b.rows, m.heads * m.dim)
-            gemm.linear(proj[nd:, o["lin_a"]:o["lin_a"] + w["a2"].shape[1]], w["a2"], out=z[nd:], bias=w["a2_bias"])
+            gemm.linear(proj[nd:, o["lin_a"]:o["lin_a"] + w["a2"].shape[1]], w["a2"], out=z[nd:], bias=w["a2_bias"], w_static=True)
             y = self.o_lin[:b.rows * n].view(b.rows, n)
             segs, seg_tokens = M.gated_linear_plan(b.n_seqs - nd, m.heads, m.vdim, b.max_q)
             M.gated_linear_prefill(proj, z, state, y, b.positions, b.slots, b.state_slots[s], b.q_starts[s], b.q_lens[s], b.max_q, self.gla_ws,
@@ -329,7 +329,7 @@ class LayeredForward:
         rows = b.rows
         proj = self.proj[:rows * lw.offs["end"]].view(rows, lw.offs["end"])
         tail = self._tail(lw, proj, rows) if self.dtype != torch.float32 else None
-        gemm.linear(x, lw.proj, out=proj, bias=lw.proj_bias, silu_cols=lw.silu_cols, tail=tail)
+        gemm.linear(x, lw.proj, out=proj, bias=lw.proj_bias, silu_cols=lw.silu_cols, tail=tail, w_static=True)
         ys, at = [], 0
         for i, m in enumerate(sub_mixers(lw.spec.mixer)):
             n = m.out_features
@@ -337,7 +337,7 @@ class LayeredForward:
             at += rows * ceil8(n)
             self._RUN[type(m)](self, l, lw, m, proj, out, b)
             y = (self.y2 if i else self.y)[:rows]
-            gemm.linear(out, lw.o_right if i else lw.o, out=y, bias=None if i else lw.o_bias)
+            gemm.linear(out, lw.o_right if i else lw.o, out=y, bias=None if i else lw.o_bias, w_static=True)
             ys.append(y)
         return proj, ys
 
@@ -375,7 +375,7 @@ class LayeredForward:
                     pending = dict(parts=self.e.port.run(l, x2, rows, mode))
                 else:
                     rg2 = self.rg2[:rows]
-                    gemm.linear(x2, lw.rg2, out=rg2, bias=lw.rg2_bias)
+                    gemm.linear(x2, lw.rg2, out=rg2, bias=lw.rg2_bias, w_static=True)
                     pending = dict(parts=self.e.port.run(l, x2, rows, mode), gate=rg2)
             if lw.side_gate is not None:
                 pending = self._token_side(l, lw, resid, x, pending)
@@ -389,7 +389,7 @@ class LayeredForward:
         M.post_norm(resid, x, **pending)
         e = self.side[:rows]
         M.gelu_gate(x, lw.side_gate, self.side_e[:rows, l * n:(l + 1) * n], e)
-        gemm.linear(e, lw.side_proj, out=self.y[:rows])
+        gemm.linear(e, lw.side_proj, out=self.y[:rows], w_static=True)
         return dict(branches=[self.y[:rows]], norm=lw.side_norm)
 
     def tap(self, layer: int, rows: int, pending: dict) -> None:
@@ -403,4 +403,4 @@ class LayeredForward:
             M.post_norm(self.resid[:rows], out[:n_sel], out_norm=e.w.final_norm, sel=sel, rows=n_sel, **self._pending)
         else:
             M.resid_norm(self.resid[:rows], e.w.final_norm, out[:n_sel], sel=sel, rows=n_sel, **self._pending)
-        gemm.linear(out[:n_sel], e.w.lm_head, out=logits[:n_sel], out_scale=e.cfg.logit_scale)
+        gemm.linear(out[:n_sel], e.w.lm_head, out=logits[:n_sel], out_scale=e.cfg.logit_scale, w_static=True)

@@ -73,6 +73,7 @@ class GemmArgs(C.Structure):
         ("tail", C.c_void_p),
         ("ld_tail", C.c_int),
         ("relu2", C.c_int),
+        ("w_static", C.c_int),
     ]
 
 

@@ -122,7 +122,8 @@ def tile_weight(w: torch.Tensor) -> TiledWeight:
 
 
 def _args(x, w, out, *, n_out, rows, epilogue, dual=0, up_offset=0, bias=None, resid=None, splits=0, bn=0,
-          num_sms=0, evict_first=None, gate_limit=0.0, up_add=0.0, act_alpha=0.0, out_scale=0.0, silu_cols=0, act_cubic=0.0) -> native.GemmArgs:
+          num_sms=0, evict_first=None, gate_limit=0.0, up_add=0.0, act_alpha=0.0, out_scale=0.0, silu_cols=0, act_cubic=0.0,
+          w_static=False) -> native.GemmArgs:
     tiled = isinstance(w, TiledWeight)
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     assert x.stride(-1) == 1 and out.stride(-1) == 1 and (tiled or w.stride(-1) == 1)
@@ -164,6 +165,7 @@ def _args(x, w, out, *, n_out, rows, epilogue, dual=0, up_offset=0, bias=None, r
     a.act_cubic = act_cubic
     a.out_scale = out_scale
     a.silu_cols = silu_cols
+    a.w_static = int(w_static)
     # decode-size calls leave room for a second kernel on the SM (the co-located Instance's attention)
     small = w.shape[0] * k * 2 <= DECODE_SMALL_WEIGHT_BYTES
     a.smem_limit = DECODE_SMEM_LIMIT if rows <= DECODE_ROWS and small else 0
@@ -188,10 +190,12 @@ def plan_shape(n_out: int, k: int, rows: int, dual: int = 0, num_sms: int = 148,
 def linear(x: torch.Tensor, w: torch.Tensor, *, out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
            resid: torch.Tensor | None = None, out_fp32: bool = False, splits: int = 0, bn: int = 0,
            num_sms: int = 0, evict_first: bool | None = None, out_scale: float = 0.0, silu_cols: int = 0,
-           tail: torch.Tensor | None = None) -> torch.Tensor:
+           tail: torch.Tensor | None = None, w_static: bool = False) -> torch.Tensor:
     """``x[rows, k] @ w[n, k].T`` (* ``out_scale`` unless 0) (+ fp32 ``bias``) (+ ``resid``) on the tcgen05 kernel; fp32
     operands run the plain fp32 kernel. The first ``silu_cols`` features are stored as ``silu(value)``. Any ``n`` and ``k``; bf16 row pitches must be multiples of 16 bytes.
-    ``tail``: the last ``tail.shape[1]`` features go to this fp32 tensor instead (bf16 products)."""
+    ``tail``: the last ``tail.shape[1]`` features go to this fp32 tensor instead (bf16 products). ``w_static``: the kernel that
+    precedes this call on the stream does not write ``w`` (true of model weights inside a forward pass), so reading it may begin
+    before that kernel ends."""
     x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])   # reshape would forget the row pitch of a single row
     rows, n = x2.shape[0], w.shape[0]
     if x.dtype == torch.float32:
@@ -205,7 +209,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, out: torch.Tensor | None = None,
         out = torch.empty(rows, n, dtype=torch.float32 if out_fp32 else torch.bfloat16, device=x.device)
     epi = EPI_STORE_F32 if out.dtype == torch.float32 else (EPI_RESIDUAL if resid is not None else EPI_STORE)
     a = _args(x2, w, out, n_out=n, rows=rows, epilogue=epi, bias=bias, resid=resid, splits=splits, bn=bn,
-              num_sms=num_sms, evict_first=evict_first, out_scale=out_scale, silu_cols=silu_cols)
+              num_sms=num_sms, evict_first=evict_first, out_scale=out_scale, silu_cols=silu_cols, w_static=w_static)
     if tail is not None:
         assert tail.dtype == torch.float32 and tail.shape[0] == rows and tail.stride(1) == 1
         a.tail, a.tail_from, a.ld_tail = tail.data_ptr(), n - tail.shape[1], tail.stride(0)
@@ -221,7 +225,8 @@ def _linear_f32(x, w, out, bias, out_scale=0.0, silu_cols=0, rows=None, n=None, 
         batch, sx, sw, so, out_scale, silu_cols, torch.cuda.current_stream(x.device).cuda_stream), "xp_gemm_f32")
 
 
-def linear_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_group_stride: int, gate: torch.Tensor | None = None) -> torch.Tensor:
+def linear_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_group_stride: int, gate: torch.Tensor | None = None,
+                   w_static: bool = False) -> torch.Tensor:
     """One small product per group (an attention head): ``x`` ``[groups, rows, k]`` with contiguous groups, ``w``
     ``[groups * n, k]``; row ``r`` of group ``g`` goes to ``out`` at element ``g * out_group_stride + r * out.stride(-2)``
     (``out`` is a view whose last dimension is at least ``n`` wide). ``gate``: logits laid out like ``out`` (a pitch of their
@@ -237,7 +242,7 @@ def linear_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_grou
             assert out.dim() == 2 and out.shape == gate.shape
             mixers.sigmoid_mul_f32(out, gate, out)
         return out
-    a = _args(x[0], w, out, n_out=n, rows=rows, epilogue=EPI_STORE if gate is None else EPI_SIGMOID, resid=gate)
+    a = _args(x[0], w, out, n_out=n, rows=rows, epilogue=EPI_STORE if gate is None else EPI_SIGMOID, resid=gate, w_static=w_static)
     a.batch, a.x_group_rows, a.w_rows_per_group, a.out_group_stride = groups, rows, n, out_group_stride
     a.ld_out = out.stride(-2)
     native.check(native.kernels().xp_gemm(C.byref(a)), "xp_gemm(batched)")
@@ -268,7 +273,8 @@ def linear_gate_mul(x: torch.Tensor, w: torch.Tensor, e: torch.Tensor, out: torc
 
 def gateup_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: torch.Tensor | None = None,
                   bias: torch.Tensor | None = None, gate_limit: float = 0.0, up_add: float = 0.0,
-                  act_alpha: float = 0.0, act_cubic: float = 0.0, splits: int = 0, bn: int = 0, num_sms: int = 0) -> torch.Tensor:
+                  act_alpha: float = 0.0, act_cubic: float = 0.0, splits: int = 0, bn: int = 0, num_sms: int = 0,
+                  w_static: bool = False) -> torch.Tensor:
     """``silu(x @ Wg.T) * (x @ Wu.T)`` with ``w_gate_up = cat([Wg, Wu])`` of shape ``[2*I, k]`` (another activation
     ``g sigmoid(act_alpha g (1 + act_cubic g^2))`` where those are given)."""
     x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
@@ -277,7 +283,7 @@ def gateup_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, *, out: torch.Tensor
     if out is None:
         out = torch.empty(rows, inter, dtype=torch.bfloat16, device=x.device)
     a = _args(x2, w_gate_up, out, n_out=inter, rows=rows, epilogue=EPI_SWIGLU, dual=1, up_offset=inter, bias=bias,
-              splits=splits, bn=bn, num_sms=num_sms, gate_limit=gate_limit, up_add=up_add, act_alpha=act_alpha, act_cubic=act_cubic)
+              splits=splits, bn=bn, num_sms=num_sms, gate_limit=gate_limit, up_add=up_add, act_alpha=act_alpha, act_cubic=act_cubic, w_static=w_static)
     native.check(native.kernels().xp_gemm(C.byref(a)), "xp_gemm(swiglu)")
     return out
 
