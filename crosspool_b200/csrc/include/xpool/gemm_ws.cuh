@@ -8,8 +8,8 @@
 // global stores are coalesced without a shared-memory transpose.
 //
 // Roles inside one 192-thread CTA:
-//   warp 0      TMA producer (one elected thread), non-multicast 2-D tile loads
-//   warp 1      TMEM allocation + tcgen05.mma issue (one elected thread)
+//   warp 0      TMA producer (one elected lane issues), non-multicast 2-D tile loads
+//   warp 1      TMEM allocation + tcgen05.mma issue (one elected lane)
 //   warps 2..5  epilogue: tcgen05.ld -> registers -> fused epilogue -> global
 // Accumulators are double-buffered in TMEM when they fit, so the epilogue of one
 // tile overlaps the main loop of the next (the CTA loops over tiles).
@@ -234,11 +234,16 @@ __device__ __forceinline__ TileCoord tile_coord(const Problem& p, int t) {
 
 // ---------------------------------------------------------------- producer
 //
-// The producer and the MMA issuer are single threads; nothing hides the latency
+// The producer and the MMA issuer are one warp each; nothing hides the latency
 // of their scalar instructions, so the per-K-block bookkeeping is kept to a few
 // adds: shared-memory addresses, barrier addresses, TMA coordinates and UMMA
 // descriptors all advance incrementally (a tcgen05.mma of N <= 32 retires in
-// about 45 cycles, four of them per K block).
+// about 45 cycles, four of them per K block). The whole warp runs the loop and
+// one elected lane issues (see elect_one): with a single thread in a branch of
+// its own a K block took 860 cycles to issue, whatever its width. One launch,
+// that form -> this one: 4096 x 1024 at 64 rows 11.1 -> 8.1 us, 151936 x 1024
+// at 32 rows 75.6 -> 53.2 us, 4096 x 12288 at 32 rows 31.2 -> 25.0 us,
+// 6144 x 4096 at 4096 rows 195 -> 183 us (bound by L2 reads of the tiles).
 
 __device__ __forceinline__ bool produce_tile(const Problem& p, const TileCoord& c,
                                              const SmemLayout& L, uint8_t* tiles, Barriers* bar,
@@ -274,21 +279,22 @@ __device__ __forceinline__ bool produce_tile(const Problem& p, const TileCoord& 
   int xc0 = c.kb0 * p.kblk;
   uint32_t stage = st.stage, phase = st.phase;
   uint32_t a_addr = tiles_addr + stage * stage_bytes;
-  const bool dual = p.dual != 0;
+  const bool dual = p.dual != 0, leader = sm100::elect_one();
   for (int i = 0; i < c.kbn; ++i) {
     const uint32_t full = full0 + stage * 8, empty = empty0 + stage * 8;
     if (i >= early) {
-      if (!sm100::mbar_try_wait_addr(empty, phase ^ 1) &&
-          !sm100::mbar_wait_addr(empty, phase ^ 1, deadline)) {
+      if (!sm100::mbar_wait_warp(empty, phase ^ 1, deadline)) {
         st.stage = stage;
         st.phase = phase;
         return false;
       }
-      sm100::mbar_arrive_expect_tx_addr(full, tx);
-      sm100::tma_load_2d_addr(a_addr, tw, full, wc0, wc1, pol_w);
-      if (dual) sm100::tma_load_2d_addr(a_addr + kTileM * kTileK * 2, tw, full, wc0, uc1, pol_w);
+      if (leader) {
+        sm100::mbar_arrive_expect_tx_addr(full, tx);
+        sm100::tma_load_2d_addr(a_addr, tw, full, wc0, wc1, pol_w);
+        if (dual) sm100::tma_load_2d_addr(a_addr + kTileM * kTileK * 2, tw, full, wc0, uc1, pol_w);
+      }
     }
-    sm100::tma_load_2d_addr(a_addr + a_bytes, tx_map, full, xc0, c.n0, pol_x);
+    if (leader) sm100::tma_load_2d_addr(a_addr + a_bytes, tx_map, full, xc0, c.n0, pol_x);
     wc0 += dwc0;
     wc1 += dwc1;
     uc1 += dwc1;
@@ -312,13 +318,16 @@ __device__ __forceinline__ int preload_weights(const Problem& p, const TileCoord
   const uint64_t tw = reinterpret_cast<uint64_t>(p.tmap_w);
   const uint32_t tiles_addr = sm100::smem_u32(tiles);
   const int n = c.kbn < L.stages ? c.kbn : L.stages, kb_total = k_blocks(p);
+  const bool leader = sm100::elect_one();
   for (int i = 0; i < n; ++i) {
     const uint32_t full = sm100::smem_u32(&bar->full[i]), dst = tiles_addr + i * L.stage_bytes;
     const int col = p.w_tiled ? 0 : (c.kb0 + i) * p.kblk;
     auto row = [&](int r) { return p.w_tiled ? ((r / kTileM) * kb_total + c.kb0 + i) * kTileM : r; };
-    sm100::mbar_arrive_expect_tx_addr(full, static_cast<uint32_t>(L.a_bytes + L.b_bytes));
-    sm100::tma_load_2d_addr(dst, tw, full, col, row(c.w_row0), pol_w);
-    if (p.dual) sm100::tma_load_2d_addr(dst + kTileM * kTileK * 2, tw, full, col, row(p.up_offset + c.w_row0), pol_w);
+    if (leader) {
+      sm100::mbar_arrive_expect_tx_addr(full, static_cast<uint32_t>(L.a_bytes + L.b_bytes));
+      sm100::tma_load_2d_addr(dst, tw, full, col, row(c.w_row0), pol_w);
+      if (p.dual) sm100::tma_load_2d_addr(dst + kTileM * kTileK * 2, tw, full, col, row(p.up_offset + c.w_row0), pol_w);
+    }
   }
   return n;
 }
@@ -349,7 +358,7 @@ __device__ __forceinline__ bool mma_tile(const Problem& p, const TileCoord& c, c
   const uint32_t tmem_g = bar->tmem_base + st.acc * acc_w;
   const uint32_t tmem_u = tmem_g + p.bn;
   const uint32_t idesc = sm100::umma_idesc_bf16(kTileM, static_cast<uint32_t>(p.bn));
-  if (!sm100::mbar_wait(&bar->acc_empty[st.acc], st.acc_phase ^ 1, deadline)) return false;
+  if (!sm100::mbar_wait_warp(sm100::smem_u32(&bar->acc_empty[st.acc]), st.acc_phase ^ 1, deadline)) return false;
   sm100::tc_fence_after_sync();
   const uint32_t tiles_addr = sm100::smem_u32(tiles);
   const uint32_t full0 = sm100::smem_u32(&bar->full[0]);
@@ -362,27 +371,29 @@ __device__ __forceinline__ bool mma_tile(const Problem& p, const TileCoord& c, c
   const uint64_t dstage = static_cast<uint64_t>(L.stage_bytes >> 4);
   uint32_t stage = st.stage, phase = st.phase;
   uint64_t da = da0 + stage * dstage, du = du0 + stage * dstage, db = db0 + stage * dstage;
-  const bool dual = p.dual != 0;
+  const bool dual = p.dual != 0, leader = sm100::elect_one();
   uint32_t accum = 0;
   for (int i = 0; i < c.kbn; ++i) {
     const uint32_t full = full0 + stage * 8;
-    if (!sm100::mbar_try_wait_addr(full, phase) && !sm100::mbar_wait_addr(full, phase, deadline)) {
+    if (!sm100::mbar_wait_warp(full, phase, deadline)) {
       st.stage = stage;
       st.phase = phase;
       return false;
     }
     sm100::tc_fence_after_sync();
     // 32 bytes (two 16-byte units) per UMMA K step inside the 128-byte swizzle row
-    sm100::umma_bf16(tmem_g, da, db, idesc, accum);
-    if (dual) sm100::umma_bf16(tmem_u, du, db, idesc, accum);
-    sm100::umma_bf16(tmem_g, da + 2, db + 2, idesc, 1u);
-    if (dual) sm100::umma_bf16(tmem_u, du + 2, db + 2, idesc, 1u);
-    sm100::umma_bf16(tmem_g, da + 4, db + 4, idesc, 1u);
-    if (dual) sm100::umma_bf16(tmem_u, du + 4, db + 4, idesc, 1u);
-    sm100::umma_bf16(tmem_g, da + 6, db + 6, idesc, 1u);
-    if (dual) sm100::umma_bf16(tmem_u, du + 6, db + 6, idesc, 1u);
+    if (leader) {
+      sm100::umma_bf16(tmem_g, da, db, idesc, accum);
+      if (dual) sm100::umma_bf16(tmem_u, du, db, idesc, accum);
+      sm100::umma_bf16(tmem_g, da + 2, db + 2, idesc, 1u);
+      if (dual) sm100::umma_bf16(tmem_u, du + 2, db + 2, idesc, 1u);
+      sm100::umma_bf16(tmem_g, da + 4, db + 4, idesc, 1u);
+      if (dual) sm100::umma_bf16(tmem_u, du + 4, db + 4, idesc, 1u);
+      sm100::umma_bf16(tmem_g, da + 6, db + 6, idesc, 1u);
+      if (dual) sm100::umma_bf16(tmem_u, du + 6, db + 6, idesc, 1u);
+      sm100::umma_commit_addr(empty0 + stage * 8);  // frees the stage when these MMAs retire
+    }
     accum = 1;
-    sm100::umma_commit_addr(empty0 + stage * 8);  // frees the stage when these MMAs retire
     da += dstage;
     du += dstage;
     db += dstage;
@@ -396,7 +407,7 @@ __device__ __forceinline__ bool mma_tile(const Problem& p, const TileCoord& c, c
   }
   st.stage = stage;
   st.phase = phase;
-  sm100::umma_commit(&bar->acc_full[st.acc]);
+  if (leader) sm100::umma_commit(&bar->acc_full[st.acc]);
   st.advance_acc(nacc);
   return true;
 }
@@ -418,10 +429,11 @@ __device__ __forceinline__ bool mma_tile_f8(const Problem& p, const TileCoord& c
   const uint64_t dstage = static_cast<uint64_t>(L.stage_bytes >> 4);
   uint32_t stage = st.stage, phase = st.phase;
   uint64_t da = da0 + stage * dstage, db = db0 + stage * dstage;
+  const bool leader = sm100::elect_one();
   for (int i = 0; i < c.kbn; ++i) {
-    if (!sm100::mbar_wait(&bar->acc_empty[st.acc], st.acc_phase ^ 1, deadline)) return false;
+    if (!sm100::mbar_wait_warp(sm100::smem_u32(&bar->acc_empty[st.acc]), st.acc_phase ^ 1, deadline)) return false;
     const uint32_t full = full0 + stage * 8;
-    if (!sm100::mbar_try_wait_addr(full, phase) && !sm100::mbar_wait_addr(full, phase, deadline)) {
+    if (!sm100::mbar_wait_warp(full, phase, deadline)) {
       st.stage = stage;
       st.phase = phase;
       return false;
@@ -429,12 +441,14 @@ __device__ __forceinline__ bool mma_tile_f8(const Problem& p, const TileCoord& c
     sm100::tc_fence_after_sync();
     const uint32_t tmem_d = bar->tmem_base + st.acc * acc_w;
     // 32 fp8 elements = 32 bytes per UMMA K step: the same descriptor stride as bf16
-    sm100::umma_f8(tmem_d, da, db, idesc, 0u);
-    sm100::umma_f8(tmem_d, da + 2, db + 2, idesc, 1u);
-    sm100::umma_f8(tmem_d, da + 4, db + 4, idesc, 1u);
-    sm100::umma_f8(tmem_d, da + 6, db + 6, idesc, 1u);
-    sm100::umma_commit_addr(empty0 + stage * 8);
-    sm100::umma_commit(&bar->acc_full[st.acc]);
+    if (leader) {
+      sm100::umma_f8(tmem_d, da, db, idesc, 0u);
+      sm100::umma_f8(tmem_d, da + 2, db + 2, idesc, 1u);
+      sm100::umma_f8(tmem_d, da + 4, db + 4, idesc, 1u);
+      sm100::umma_f8(tmem_d, da + 6, db + 6, idesc, 1u);
+      sm100::umma_commit_addr(empty0 + stage * 8);
+      sm100::umma_commit(&bar->acc_full[st.acc]);
+    }
     st.advance_acc(nacc);
     da += dstage;
     db += dstage;

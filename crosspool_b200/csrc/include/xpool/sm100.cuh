@@ -31,6 +31,22 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a converged warp. Loops that issue TMA copies or tcgen05 instructions are run by the whole warp, with only the
+// issuing instructions predicated by this: descriptors, coordinates and addresses then live in uniform registers, where those
+// instructions want them. (In a branch that only lane 0 takes, every operand is moved over one by one: four tcgen05.mma took
+// 507 cycles to issue.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -407,6 +423,10 @@ static __device__ __noinline__ bool mbar_wait_addr(uint32_t bar, uint32_t parity
     if ((++spins & 0x3ffu) == 0 && global_timer_ns() > deadline_ns) return false;
   }
   return true;
+}
+// As mbar_wait, for a converged warp: every lane waits and all leave with the same answer, also where the limit runs out.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint64_t deadline_ns) {
+  return __all_sync(0xffffffffu, mbar_try_wait_addr(bar, parity) || mbar_wait_addr(bar, parity, deadline_ns));
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx_addr(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");

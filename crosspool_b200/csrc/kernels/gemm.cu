@@ -26,7 +26,7 @@ __device__ __forceinline__ void run_tiles(const Problem& p, int nacc, int smem_b
   // Set-up and the first weight tiles do not depend on the stream's previous kernel; everything below does (the Lane form is
   // an ordinary launch, where the wait returns at once).
   int early = 0;
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     sm100::tma_prefetch_desc(p.tmap_w);
     sm100::tma_prefetch_desc(p.tmap_x);
     if (p.w_static && p.tile_table == nullptr && static_cast<int>(blockIdx.x) < tile_count(p))
@@ -37,29 +37,24 @@ __device__ __forceinline__ void run_tiles(const Problem& p, int nacc, int smem_b
   const int ntiles = tile_count(p);
 
   if (warp == 0) {
-    if (lane == 0) {
-      PipeState st;
-      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint64_t deadline = sm100::global_timer_ns() + sm100::kPipelineWaitNs;
-        if (!produce_tile(p, tile_coord(p, t), L, tiles, bar, st, deadline, t == static_cast<int>(blockIdx.x) ? early : 0)) {
-          record_status(status, kTimeoutProducer);
-          producer_drain(L, bar, st);
-          break;
-        }
+    PipeState st;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const uint64_t deadline = sm100::global_timer_ns() + sm100::kPipelineWaitNs;
+      if (!produce_tile(p, tile_coord(p, t), L, tiles, bar, st, deadline, t == static_cast<int>(blockIdx.x) ? early : 0)) {
+        record_status(status, kTimeoutProducer);
+        producer_drain(L, bar, st);
+        break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      PipeState st;
-      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint64_t deadline = sm100::global_timer_ns() + sm100::kPipelineWaitNs;
-        if (!mma_tile(p, tile_coord(p, t), L, tiles, bar, st, nacc, deadline)) {
-          record_status(status, kTimeoutMma);
-          break;
-        }
+    PipeState st;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const uint64_t deadline = sm100::global_timer_ns() + sm100::kPipelineWaitNs;
+      if (!mma_tile(p, tile_coord(p, t), L, tiles, bar, st, nacc, deadline)) {
+        record_status(status, kTimeoutMma);
+        break;
       }
     }
-    __syncwarp();
   } else {
     PipeState st;
     const int ew = warp & 3;
