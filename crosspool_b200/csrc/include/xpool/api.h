@@ -95,7 +95,7 @@ typedef struct XpNormArgs {
   void* trace_events;
   void* trace_state;
   uint32_t trace_capacity;
-  uint32_t reserved;
+  uint32_t w_static;           /* the kernel before this call on the stream does not write weight (model weights) */
 } XpNormArgs;
 
 /* Attention side: wait (bounded) until each flag reaches *want_ptr (or `want`). */

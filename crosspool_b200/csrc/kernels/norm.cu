@@ -41,14 +41,127 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return t;
 }
 
-// One CTA per row; hidden % 8 == 0; hidden <= 8 * kThreads * kMaxVec.
 constexpr int kMaxVec = 4;  // 256 threads * 8 elems * 4 = 8192 hidden max
+
+__device__ __forceinline__ void add8(float (&acc)[8], const uint4& raw) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = __bfloat1622float2(h[j]);
+    acc[2 * j] += f.x;
+    acc[2 * j + 1] += f.y;
+  }
+}
+
+// The same arithmetic, in the same order of sums, for rows that neither wait for another GPU nor are sent to one. What bounds it
+// is one round of loads: inputs, residual and weights of a row are requested together (the weights, where they are the
+// model's, before the previous kernel has ended; in a decode step they come from HBM). kWarp: rows of at most 1024 elements are a
+// warp's, eight rows a CTA, and need no block barrier; wider ones are a CTA's. Beside the general kernel:
+// 6000 rows of 4096 54.4 -> 41.1 us (196 MB: 4.8 TB/s).
+template <bool kWarp>
+__global__ void __launch_bounds__(kThreads)
+norm_rows_kernel(XpNormArgs a) {
+  __shared__ float red[kThreads / 32];
+  const int lane = threadIdx.x & 31;
+  const int row = kWarp ? blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5) : blockIdx.x;
+  const int first = kWarp ? lane : threadIdx.x, step = kWarp ? 32 : kThreads;
+  const int nvec = a.hidden / 8;
+  uint4 w[kMaxVec], x[kMaxVec], r[kMaxVec];
+  auto load_weight = [&] {
+#pragma unroll
+    for (int it = 0; it < kMaxVec; ++it)
+      if (first + it * step < nvec) w[it] = reinterpret_cast<const uint4*>(a.weight)[first + it * step];
+  };
+  if (a.weight != nullptr && a.w_static) load_weight();
+  pdl::wait();
+  pdl::release();
+  if (row >= a.rows) return;     // (whole warps or nobody)
+  auto part = [&](int p, int v) {
+    return __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.parts[p]) + static_cast<size_t>(row) * a.ld_parts) + v);
+  };
+  uint4* resid = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.resid) + static_cast<size_t>(row) * a.hidden);
+#pragma unroll
+  for (int it = 0; it < kMaxVec; ++it) {
+    const int v = first + it * step;
+    if (v < nvec) {
+      x[it] = part(0, v);
+      if (a.resid != nullptr) r[it] = resid[v];
+    }
+  }
+  if (a.weight != nullptr && !a.w_static) load_weight();
+  float vals[kMaxVec][8], ss[kMaxVec];
+#pragma unroll
+  for (int it = 0; it < kMaxVec; ++it) {
+    ss[it] = 0.f;
+    const int v = first + it * step;
+    if (v >= nvec) continue;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    add8(acc, x[it]);
+    for (int p = 1; p < a.nparts; ++p) add8(acc, part(p, v));
+    if (a.nparts > 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = __bfloat162float(__float2bfloat16_rn(acc[j]));
+    }
+    if (a.resid != nullptr) {
+      add8(acc, r[it]);
+      Bf16x8 y;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        y.v[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+        const float2 b = __bfloat1622float2(y.v[j]);
+        acc[2 * j] = b.x;
+        acc[2 * j + 1] = b.y;
+      }
+      resid[v] = *reinterpret_cast<const uint4*>(&y);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      vals[it][j] = acc[j];
+      ss[it] = fmaf(acc[j], acc[j], ss[it]);
+    }
+  }
+  if (a.weight == nullptr) return;
+  float total;
+  if (kWarp) {
+    // the sums of the four warps that would share the row in a CTA, added as block_sum adds them
+    static_assert(kMaxVec == 4, "a tree of four");
+#pragma unroll
+    for (int it = 0; it < kMaxVec; ++it) ss[it] = warp_sum(ss[it]);
+    total = (ss[0] + ss[2]) + (ss[1] + ss[3]);
+  } else {
+    float t = 0.f;
+#pragma unroll
+    for (int it = 0; it < kMaxVec; ++it)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (first + it * step < nvec) t = fmaf(vals[it][j], vals[it][j], t);
+    total = block_sum(t, red);
+  }
+  const float inv = rsqrtf(total / static_cast<float>(a.hidden) + a.eps);
+  uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out_local) + static_cast<size_t>(row) * a.ld_out);
+#pragma unroll
+  for (int it = 0; it < kMaxVec; ++it) {
+    const int v = first + it * step;
+    if (v >= nvec) continue;
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w[it]);
+    Bf16x8 y;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 wf = __bfloat1622float2(h[j]);
+      const float n0 = __bfloat162float(__float2bfloat16_rn(vals[it][2 * j] * inv));
+      const float n1 = __bfloat162float(__float2bfloat16_rn(vals[it][2 * j + 1] * inv));
+      y.v[j] = __floats2bfloat162_rn(n0 * wf.x, n1 * wf.y);
+    }
+    if (a.out_local != nullptr) out[v] = *reinterpret_cast<const uint4*>(&y);
+  }
+}
+
+// General form: one CTA per row; hidden % 8 == 0; hidden <= 8 * kThreads * kMaxVec.
 
 __global__ void __launch_bounds__(kThreads)
 norm_publish_kernel(XpNormArgs a) {
   // A CTA that may spin on another GPU's flag holds its successor back: CTAs resident early would take the room of what it waits for.
   pdl::wait();
-  if (a.wait_seq == 0 && a.npeers == 0) pdl::release();
   __shared__ float red[kThreads / 32];
   __shared__ uint32_t s_fail;
   const int row = blockIdx.x;
@@ -210,6 +323,14 @@ swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ 
 extern "C" int xp_norm_publish(const XpNormArgs* a, void* stream) {
   if (a->hidden % 8 != 0 || a->hidden > 8 * xpool::norm::kThreads * xpool::norm::kMaxVec) return -10;
   if (a->rows <= 0 || a->nparts < 1 || a->nparts > 8 || a->npeers < 0 || a->npeers > 8) return -11;
+  if (a->wait_seq == 0 && a->npeers == 0) {
+    using namespace xpool::norm;
+    const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (a->hidden <= 1024) xpool::pdl::launch(norm_rows_kernel<true>, (a->rows + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, s, 1, *a);
+    else xpool::pdl::launch(norm_rows_kernel<false>, a->rows, kThreads, 0, s, 1, *a);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
+  }
   xpool::pdl::launch(xpool::norm::norm_publish_kernel, a->rows, xpool::norm::kThreads, 0, reinterpret_cast<cudaStream_t>(stream), 1, *a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);

@@ -13,73 +13,111 @@
 namespace xpool {
 namespace rope {
 
-template <int D>
+constexpr int kHeadsInFlight = 4;
+
+// A warp takes every heads_step-th head of a row: the angles are the row's, so their sines are computed once a warp (they were
+// most of the work when every head had a warp of its own), and the loads of four heads are in flight together. Lane l
+// rotates elements l PER .. + PER - 1 of one half with those of the other. WIDE: pairs of elements are 4-byte aligned.
+// 4096 rows of 32 heads of 128: 29.6 -> 26.6 us.
+template <int D, bool WIDE>
 __global__ void __launch_bounds__(256)
-rope_kv_kernel(XpRopeArgs a) {
-  pdl::wait();
-  pdl::release();
+rope_kv_kernel(XpRopeArgs a, int heads_step) {
   constexpr int PER = D / 64;  // elements per lane in each half
   const int row = blockIdx.x;
-  const int head = blockIdx.y * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const int heads_total = a.q_heads + 2 * a.kv_heads;
-  if (head >= heads_total) return;
-  const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.qkv) +
-                             static_cast<size_t>(row) * a.ld_qkv + static_cast<size_t>(head) * D;
-  const bool is_q = head < a.q_heads;
-  const bool is_k = !is_q && head < a.q_heads + a.kv_heads;
-  float x1[PER], x2[PER];
+  const int first = blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int heads_total = a.q_heads + 2 * a.kv_heads, rotated = a.q_heads + a.kv_heads;
+  auto load = [&](const __nv_bfloat16* p, float (&v)[PER]) {
+    if constexpr (WIDE && PER == 2) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + lane * PER));
+      v[0] = f.x, v[1] = f.y;
+    } else {
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    x1[i] = __bfloat162float(src[lane * PER + i]);
-    x2[i] = __bfloat162float(src[D / 2 + lane * PER + i]);
-  }
-  if (is_q || is_k) {
-    const __nv_bfloat16* nw =
-        reinterpret_cast<const __nv_bfloat16*>(is_q ? a.q_norm_weight : a.k_norm_weight);
-    if (nw != nullptr) {
-      float ss = 0.f;
+      for (int i = 0; i < PER; ++i) v[i] = __bfloat162float(p[lane * PER + i]);
+    }
+  };
+  auto store = [&](__nv_bfloat16* p, const float (&v)[PER]) {
+    if constexpr (WIDE && PER == 2) {
+      *reinterpret_cast<__nv_bfloat162*>(p + lane * PER) = __floats2bfloat162_rn(v[0], v[1]);
+    } else {
 #pragma unroll
-      for (int i = 0; i < PER; ++i) ss += x1[i] * x1[i] + x2[i] * x2[i];
+      for (int i = 0; i < PER; ++i) p[lane * PER + i] = __float2bfloat16_rn(v[i]);
+    }
+  };
+  pdl::wait();
+  pdl::release();
+  if (first >= heads_total) return;
+  const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.qkv) + static_cast<size_t>(row) * a.ld_qkv;
+  const __nv_bfloat16* qn = reinterpret_cast<const __nv_bfloat16*>(a.q_norm_weight);
+  const __nv_bfloat16* kn = reinterpret_cast<const __nv_bfloat16*>(a.k_norm_weight);
+  const int slot = a.slots[row];
+  const float pos = static_cast<float>(a.positions[row]);
+  float c[PER], s[PER];
+  bool have = false;
+  for (int h0 = first; h0 < heads_total; h0 += kHeadsInFlight * heads_step) {
+    float x1[kHeadsInFlight][PER], x2[kHeadsInFlight][PER], n1[kHeadsInFlight][PER], n2[kHeadsInFlight][PER];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float inv = rsqrtf(ss / D + a.eps);
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        float n1 = __bfloat162float(__float2bfloat16_rn(x1[i] * inv));
-        float n2 = __bfloat162float(__float2bfloat16_rn(x2[i] * inv));
-        x1[i] = __bfloat162float(__float2bfloat16_rn(n1 * __bfloat162float(nw[lane * PER + i])));
-        x2[i] = __bfloat162float(__float2bfloat16_rn(n2 * __bfloat162float(nw[D / 2 + lane * PER + i])));
+    for (int u = 0; u < kHeadsInFlight; ++u) {
+      const int head = h0 + u * heads_step;
+      if (head < heads_total) {
+        load(src + static_cast<size_t>(head) * D, x1[u]);
+        load(src + static_cast<size_t>(head) * D + D / 2, x2[u]);
+        const __nv_bfloat16* nw = head < a.q_heads ? qn : head < rotated ? kn : nullptr;
+        if (nw != nullptr) {
+          load(nw, n1[u]);
+          load(nw + D / 2, n2[u]);
+        }
       }
     }
-    const float pos = static_cast<float>(a.positions[row]);
+    if (!have && h0 < rotated) {      // beside the loads
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int idx = lane * PER + i;
-      const float inv_freq = exp2f(-(2.f * idx / D) * a.log2_theta);
-      float s, c;
-      sincosf(pos * inv_freq, &s, &c);
-      const float r1 = x1[i] * c - x2[i] * s;
-      const float r2 = x2[i] * c + x1[i] * s;
-      x1[i] = r1;
-      x2[i] = r2;
+      for (int i = 0; i < PER; ++i) {
+        const int idx = lane * PER + i;
+        const float inv_freq = exp2f(-(2.f * idx / D) * a.log2_theta);
+        sincosf(pos * inv_freq, &s[i], &c[i]);
+      }
+      have = true;
     }
-  }
-  __nv_bfloat16* dst;
-  if (is_q) {
-    dst = reinterpret_cast<__nv_bfloat16*>(a.q_out) + static_cast<size_t>(row) * a.q_heads * D +
-          static_cast<size_t>(head) * D;
-  } else {
-    const int slot = a.slots[row];
-    if (slot < 0) return;
-    const int hk = is_k ? head - a.q_heads : head - a.q_heads - a.kv_heads;
-    __nv_bfloat16* cache = reinterpret_cast<__nv_bfloat16*>(is_k ? a.k_cache : a.v_cache);
-    dst = cache + (static_cast<size_t>(slot) * a.kv_heads + hk) * D;
-  }
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    dst[lane * PER + i] = __float2bfloat16_rn(x1[i]);
-    dst[D / 2 + lane * PER + i] = __float2bfloat16_rn(x2[i]);
+    for (int u = 0; u < kHeadsInFlight; ++u) {
+      const int head = h0 + u * heads_step;
+      if (head >= heads_total) break;
+      const bool is_q = head < a.q_heads;
+      if (head < rotated) {
+        if ((is_q ? qn : kn) != nullptr) {
+          float ss = 0.f;
+#pragma unroll
+          for (int i = 0; i < PER; ++i) ss += x1[u][i] * x1[u][i] + x2[u][i] * x2[u][i];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+          const float inv = rsqrtf(ss / D + a.eps);
+#pragma unroll
+          for (int i = 0; i < PER; ++i) {
+            const float v1 = __bfloat162float(__float2bfloat16_rn(x1[u][i] * inv));
+            const float v2 = __bfloat162float(__float2bfloat16_rn(x2[u][i] * inv));
+            x1[u][i] = __bfloat162float(__float2bfloat16_rn(v1 * n1[u][i]));
+            x2[u][i] = __bfloat162float(__float2bfloat16_rn(v2 * n2[u][i]));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          const float r1 = x1[u][i] * c[i] - x2[u][i] * s[i];
+          const float r2 = x2[u][i] * c[i] + x1[u][i] * s[i];
+          x1[u][i] = r1;
+          x2[u][i] = r2;
+        }
+      }
+      __nv_bfloat16* dst;
+      if (is_q) {
+        dst = reinterpret_cast<__nv_bfloat16*>(a.q_out) + (static_cast<size_t>(row) * a.q_heads + head) * D;
+      } else {
+        if (slot < 0) continue;
+        const int hk = head < rotated ? head - a.q_heads : head - rotated;
+        dst = reinterpret_cast<__nv_bfloat16*>(head < rotated ? a.k_cache : a.v_cache) + (static_cast<size_t>(slot) * a.kv_heads + hk) * D;
+      }
+      store(dst, x1[u]);
+      store(dst + D / 2, x2[u]);
+    }
   }
 }
 
@@ -89,12 +127,20 @@ rope_kv_kernel(XpRopeArgs a) {
 extern "C" int xp_rope_kv(const XpRopeArgs* a, void* stream) {
   if (a->rows <= 0) return 0;
   const int heads_total = a->q_heads + 2 * a->kv_heads;
-  dim3 grid(a->rows, (heads_total + 7) / 8);
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (a->head_dim == 128)
-    xpool::pdl::launch(xpool::rope::rope_kv_kernel<128>, grid, 256, 0, s, 1, *a);
+  // A CTA per row where the rows alone fill the SMs several times over; in a decode step every head has a warp.
+  const bool many = a->rows >= 148 * 4;
+  const dim3 grid(a->rows, many ? 1 : (heads_total + 7) / 8);
+  const int step = static_cast<int>(grid.y) * 8;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  auto pair = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3) == 0; };
+  const bool wide = a->ld_qkv % 2 == 0 && pair(a->qkv) && pair(a->q_out) && pair(a->k_cache) && pair(a->v_cache) && pair(a->q_norm_weight) && pair(a->k_norm_weight);
+  using namespace xpool::rope;
+  if (a->head_dim == 128 && wide)
+    xpool::pdl::launch(rope_kv_kernel<128, true>, grid, 256, 0, s, 1, *a, step);
+  else if (a->head_dim == 128)
+    xpool::pdl::launch(rope_kv_kernel<128, false>, grid, 256, 0, s, 1, *a, step);
   else if (a->head_dim == 64)
-    xpool::pdl::launch(xpool::rope::rope_kv_kernel<64>, grid, 256, 0, s, 1, *a);
+    xpool::pdl::launch(rope_kv_kernel<64, true>, grid, 256, 0, s, 1, *a, step);
   else
     return -10;
   cudaError_t e = cudaGetLastError();

@@ -347,9 +347,9 @@ class AttentionEngine:
         parts: list[torch.Tensor] | None = None
         for l, lw in enumerate(w.layers):
             if parts is None:
-                norm.add_rmsnorm([resid], lw.input_norm, cfg.rms_norm_eps, out=x)
+                norm.add_rmsnorm([resid], lw.input_norm, cfg.rms_norm_eps, out=x, w_static=True)
             else:
-                norm.add_rmsnorm(weight=lw.input_norm, eps=cfg.rms_norm_eps, resid=resid, out=x, **_parts_kw(parts),
+                norm.add_rmsnorm(weight=lw.input_norm, eps=cfg.rms_norm_eps, resid=resid, out=x, w_static=True, **_parts_kw(parts),
                                  **self.port.wait_args())
             gemm.linear(x, lw.qkv, out=self.qkv[:rows], bias=lw.qkv_bias, w_static=True)
             attn_fn(l, lw, rows)
@@ -363,7 +363,7 @@ class AttentionEngine:
                 self.tp.exchange()
                 o_parts = dict(parts=[], part_ptrs=self.tp.part_ptrs(l), part_shape=(rows, cfg.hidden_size, cfg.hidden_size))
             if tgt is None:
-                norm.add_rmsnorm(weight=lw.post_attn_norm, eps=cfg.rms_norm_eps, resid=resid, out=x2, **o_parts)
+                norm.add_rmsnorm(weight=lw.post_attn_norm, eps=cfg.rms_norm_eps, resid=resid, out=x2, w_static=True, **o_parts)
             else:
                 norm.add_rmsnorm(weight=lw.post_attn_norm, eps=cfg.rms_norm_eps, resid=resid, out=x2,
                                  want_local=False, **tgt, **o_parts)
@@ -373,7 +373,7 @@ class AttentionEngine:
     def _head(self, rows: int, n_sel: int, sel_idx: torch.Tensor | None) -> None:
         """Final norm, row selection, LM head, greedy sampling into ``self.tokens[:n_sel]``."""
         cfg = self.cfg
-        norm.add_rmsnorm(weight=self.w.final_norm, eps=cfg.rms_norm_eps, resid=self.resid[:rows], out=self.x[:rows],
+        norm.add_rmsnorm(weight=self.w.final_norm, eps=cfg.rms_norm_eps, resid=self.resid[:rows], out=self.x[:rows], w_static=True,
                          **_parts_kw(self._parts),
                          **self.port.wait_args())
         if sel_idx is None:

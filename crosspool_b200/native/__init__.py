@@ -123,7 +123,7 @@ class NormArgs(C.Structure):
         ("trace_events", C.c_void_p),
         ("trace_state", C.c_void_p),
         ("trace_capacity", C.c_uint32),
-        ("reserved", C.c_uint32),
+        ("w_static", C.c_uint32),
     ]
 
 

@@ -36,7 +36,8 @@ def add_rmsnorm(parts: Sequence[torch.Tensor] | torch.Tensor, weight: torch.Tens
                 wait_ns: int = 5_000_000_000, meta: tuple[int, int, int] = (0, 0, 0),
                 want_local: bool = True, seq_counter_ptr: int = 0,
                 part_ptrs: Sequence[int] | None = None, part_shape: tuple[int, int, int] | None = None,
-                deadline_ptr: int = 0, cancel_ptr: int = 0, trace: tuple[int, int, int] | None = None) -> torch.Tensor | None:
+                deadline_ptr: int = 0, cancel_ptr: int = 0, trace: tuple[int, int, int] | None = None,
+                w_static: bool = False) -> torch.Tensor | None:
     """``y = rmsnorm(sum(parts) + resid) * weight``; ``resid`` is updated in place.
 
     ``parts`` are bf16 ``[rows, hidden]`` tensors summed in list order. Parts that live in another
@@ -44,7 +45,8 @@ def add_rmsnorm(parts: Sequence[torch.Tensor] | torch.Tensor, weight: torch.Tens
     ``part_shape = (rows, hidden, leading dimension)``; the device then comes from ``resid``/``out``.
     With ``weight=None`` only the residual add happens. ``cancel_ptr``: a device word that ends the waits when it
     turns non-zero (the claim word of the Instance's failure slot). ``trace``: (events, state, capacity) of a device
-    event buffer the kernel's hook points record into.
+    event buffer the kernel's hook points record into. ``w_static``: the kernel that precedes this call on the stream does not
+    write ``weight`` (true of model weights inside a forward pass).
     """
     if isinstance(parts, torch.Tensor):
         parts = [parts]
@@ -86,6 +88,7 @@ def add_rmsnorm(parts: Sequence[torch.Tensor] | torch.Tensor, weight: torch.Tens
     a.wait_seq, a.publish_seq = wait_seq, publish_seq
     a.meta_layer, a.meta_mode, a.meta_deadline_us = meta
     a.eps = eps
+    a.w_static = int(w_static)
     a.seq_counter = seq_counter_ptr or None
     a.meta_deadline_ptr = deadline_ptr or None
     native.check(native.kernels().xp_norm_publish(C.byref(a), torch.cuda.current_stream(dev).cuda_stream),
