@@ -247,9 +247,12 @@ struct TileChoice {
 
 static TileChoice choose_tiles(int tm, int rows, int kb, int dual, int sms, int fixed_bn, int fixed_splits,
                                size_t ws_bytes_available, int max_bn = 256) {
-  // 256-wide dual tiles use all 512 TMEM columns (one accumulator buffer, no epilogue overlap): worth it
-  // only when they make the activation a single tile, so that every weight byte is fetched once
-  const int cap = std::min((dual && fixed_bn != 256 && !(rows > 128 && rows <= 256)) ? 128 : 256, max_bn);
+  // 256-wide dual tiles use all 512 TMEM columns (one accumulator buffer, no epilogue overlap). They pay where the activation is
+  // a single tile, so that every weight byte is fetched once, and where K is long: 64 KB of operands per 256 x 256 products
+  // of a K block instead of 96, against an epilogue of about 14 us a tile. gate/up at 4096 rows, 128 -> 256 wide: K = 1024 53.5 -> 71.1
+  // us, K = 4096 891 -> 704 us; 1000 rows K = 4096 224 -> 181 us.
+  const bool long_k = kb >= 32 && rows > 256;
+  const int cap = std::min((dual && fixed_bn != 256 && !long_k && !(rows > 128 && rows <= 256)) ? 128 : 256, max_bn);
   int top = 16;
   while (top < rows && top < cap) top <<= 1;
   TileChoice best{top, 1};
@@ -258,6 +261,7 @@ static TileChoice choose_tiles(int tm, int rows, int kb, int dual, int sms, int 
   for (int bn = 16; bn <= top; bn <<= 1) {
     if (fixed_bn > 0 && bn != fixed_bn) continue;
     if (fixed_bn <= 0 && bn * 4 < top && bn < 64) continue;  // no forests of tiny tiles
+    if (fixed_bn <= 0 && dual && long_k && bn < 256 && (rows + 255) / 256 * 256 * 10 <= (rows + 127) / 128 * 128 * 11) continue;
     const int tn = (rows + bn - 1) / bn;
     for (int s : kSplits) {
       if (fixed_splits > 0 && s != fixed_splits) continue;
