@@ -609,6 +609,48 @@ __device__ __forceinline__ void epilogue_store16(const Problem& p, int f, int fb
   }
 }
 
+// Columns [lo, hi) of a finished accumulator (hi - lo > 0 where anything is to be stored). Two register buffers: the TMEM read of the
+// next 16 columns is in flight while the current ones go through the epilogue math and their stores. All conditions are
+// warp-uniform.
+template <bool kWide>
+__device__ __forceinline__ void epilogue_columns(const Problem& p, const TileCoord& c, int f, int fb, uint32_t tmem_acc, int lo, int hi, bool wide) {
+  if (lo >= hi) return;
+  float g[16], u[16];
+  const uint32_t up = tmem_acc + static_cast<uint32_t>(p.bn);
+  uint32_t ga[16], ua[16], gb[16], ub[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) ua[j] = ub[j] = 0u;
+  sm100::tmem_ld16_issue(tmem_acc + lo, ga);
+  if (p.dual) sm100::tmem_ld16_issue(up + lo, ua);
+  for (int col = lo; col < hi; col += 32) {
+    sm100::tmem_ld_wait32(ga, ua);
+    const bool more = col + 16 < hi;
+    if (more) {
+      sm100::tmem_ld16_issue(tmem_acc + col + 16, gb);
+      if (p.dual) sm100::tmem_ld16_issue(up + col + 16, ub);
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      g[j] = __uint_as_float(ga[j]);
+      u[j] = __uint_as_float(ua[j]);
+    }
+    epilogue_store16<kWide>(p, f, fb, c.n0 + col, c.row_end, g, u, c.out_off, wide);
+    if (more) {
+      sm100::tmem_ld_wait32(gb, ub);
+      if (col + 32 < hi) {
+        sm100::tmem_ld16_issue(tmem_acc + col + 32, ga);
+        if (p.dual) sm100::tmem_ld16_issue(up + col + 32, ua);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        g[j] = __uint_as_float(gb[j]);
+        u[j] = __uint_as_float(ub[j]);
+      }
+      epilogue_store16<kWide>(p, f, fb, c.n0 + col + 16, c.row_end, g, u, c.out_off, wide);
+    }
+  }
+}
+
 // Runs on the 128 epilogue threads. `ew` is the warp's TMEM lane quarter.
 template <bool kWide>
 __device__ __forceinline__ bool epilogue_tile(const Problem& p, const TileCoord& c, Barriers* bar,
@@ -694,42 +736,7 @@ __device__ __forceinline__ bool epilogue_tile(const Problem& p, const TileCoord&
         if (j < p.bn) ws[static_cast<size_t>(j) * kTileM + lane_in_tile] = acc[j];
     }
   } else if (p.splits == 1) {
-    // Two register buffers: the TMEM read of the next 16 columns is in flight while the current
-    // ones go through the epilogue math and their stores. All conditions are warp-uniform.
-    const int ncol = min(p.bn, c.row_end - c.n0);  // columns that hold rows to store (> 0)
-    const uint32_t up = tmem_acc + static_cast<uint32_t>(p.bn);
-    uint32_t ga[16], ua[16], gb[16], ub[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) ua[j] = ub[j] = 0u;
-    sm100::tmem_ld16_issue(tmem_acc, ga);
-    if (p.dual) sm100::tmem_ld16_issue(up, ua);
-    for (int col = 0; col < ncol; col += 32) {
-      sm100::tmem_ld_wait32(ga, ua);
-      const bool more = col + 16 < ncol;
-      if (more) {
-        sm100::tmem_ld16_issue(tmem_acc + col + 16, gb);
-        if (p.dual) sm100::tmem_ld16_issue(up + col + 16, ub);
-      }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        g[j] = __uint_as_float(ga[j]);
-        u[j] = __uint_as_float(ua[j]);
-      }
-      epilogue_store16<kWide>(p, f, fb, c.n0 + col, c.row_end, g, u, c.out_off, wide);
-      if (more) {
-        sm100::tmem_ld_wait32(gb, ub);
-        if (col + 32 < ncol) {
-          sm100::tmem_ld16_issue(tmem_acc + col + 32, ga);
-          if (p.dual) sm100::tmem_ld16_issue(up + col + 32, ua);
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          g[j] = __uint_as_float(gb[j]);
-          u[j] = __uint_as_float(ub[j]);
-        }
-        epilogue_store16<kWide>(p, f, fb, c.n0 + col + 16, c.row_end, g, u, c.out_off, wide);
-      }
-    }
+    epilogue_columns<kWide>(p, c, f, fb, tmem_acc, 0, min(p.bn, c.row_end - c.n0), wide);
   } else {
     // Split-K: park raw partial sums, last-arriving CTA folds them in split order.
     float* ws = p.ws + (static_cast<size_t>(c.mn) * p.splits + c.split) * acc_cols * kTileM;

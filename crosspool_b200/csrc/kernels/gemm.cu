@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "xpool/api.h"
+#include "xpool/gemm_pair.cuh"
 #include "xpool/gemm_stream.cuh"
 #include "xpool/gemm_ws.cuh"
 #include "xpool/lane.cuh"
@@ -417,6 +418,14 @@ extern "C" int xp_gemm(const XpGemmArgs* a) {
   p.ld_tail = a->ld_tail;
   p.relu2 = a->relu2;
   p.w_static = a->w_static;
+  const bool wide = p.act_cubic != 0.f || p.epilogue == gemm::kEpiGateMul || p.epilogue == gemm::kEpiSigmoid || p.tail != nullptr || p.relu2 != 0;
+  {
+    int d = 0, sms = 148;
+    cudaGetDevice(&d);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
+    const int width = gemm::pair_width(*a, sms);
+    if (width > 0) return gemm::pair_launch(*a, p, tw, width, wide, sms);
+  }
   if (a->tile_table != nullptr) {
     if (plan.splits != 1) return -13;
     plan.grid = plan.smem_bytes > 0 ? 148 : 148;
@@ -435,7 +444,6 @@ extern "C" int xp_gemm(const XpGemmArgs* a) {
       return -30;
     attr_set[dev] = true;
   }
-  const bool wide = p.act_cubic != 0.f || p.epilogue == gemm::kEpiGateMul || p.epilogue == gemm::kEpiSigmoid || p.tail != nullptr || p.relu2 != 0;
   auto kernel = wide ? gemm::gemm_ws_kernel<true> : gemm::gemm_ws_kernel<false>;
   pdl::launch(kernel, plan.grid, gemm::kThreads, plan.smem_bytes, reinterpret_cast<cudaStream_t>(a->stream), 1, tw, tx, p, plan.nacc, plan.smem_budget, a->status);
   cudaError_t e = cudaGetLastError();

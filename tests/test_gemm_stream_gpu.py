@@ -40,7 +40,9 @@ def test_epilogues(rows):
     r = torch.randn(rows, n, device="cuda", generator=g).bfloat16()
     y = x.float() @ w.float().t()
     _close(gemm.linear(x, w, bias=b, out_scale=0.5), y * 0.5 + b)
-    _close(gemm.linear(x, w, resid=r), y.bfloat16().float() + r.float(), 2)
+    # the product is rounded before the sum: where its order of sums flips that rounding, the sum is off by a unit of the product
+    got, want = gemm.linear(x, w, resid=r).float(), y.bfloat16().float() + r.float()
+    assert ((got - want).abs() <= 2.0 ** -7 * y.abs() + 2.0 ** -8 * want.abs() + 1e-5).all()
     got = gemm.linear(x, w, silu_cols=50)
     _close(got, torch.cat([torch.nn.functional.silu(y[:, :50]), y[:, 50:]], 1))
     out, tail = torch.empty(rows, n, device="cuda", dtype=torch.bfloat16), torch.empty(rows, 7, device="cuda")
