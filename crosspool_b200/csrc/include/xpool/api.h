@@ -62,6 +62,7 @@ typedef struct XpGemmArgs {
   int ld_tail;
   int relu2;           /* epilogue 0: values are stored as max(value, 0)^2 */
   int w_static;        /* the kernel before this call on the stream does not write w (model weights): it may be read early */
+  int tile_pairs;      /* entries 2 j and 2 j + 1 of the tile table are neighbouring feature tiles of one group and row tile */
 } XpGemmArgs;
 
 typedef struct XpGemmPlan {

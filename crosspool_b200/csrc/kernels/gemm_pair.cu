@@ -39,16 +39,24 @@ __host__ __device__ inline PairLayout pair_layout(int bn, int dual) {
 // Tile t of the pair: CTA `rank` owns weight rows m0 .. + 127; the activation rows are the pair's.
 __device__ __forceinline__ TileCoord pair_coord(const Problem& p, int t, int rank) {
   TileCoord c;
-  const int tm = (p.n_out + 2 * kTileM - 1) / (2 * kTileM);
-  c.m0 = (t % tm) * 2 * kTileM + rank * kTileM;
-  c.n0 = (t / tm) * p.bn;
   c.split = 0;
   c.mn = t;
   c.kb0 = 0;
   c.kbn = k_blocks(p);
+  c.out_off = 0;
+  if (p.tile_table != nullptr) {
+    const int4 e = p.tile_table[2 * t + rank];
+    c.m0 = e.y;
+    c.n0 = e.z;
+    c.row_end = e.w;
+    c.w_row0 = e.x * p.w_rows_per_group + e.y;
+    return c;
+  }
+  const int tm = (p.n_out + 2 * kTileM - 1) / (2 * kTileM);
+  c.m0 = (t % tm) * 2 * kTileM + rank * kTileM;
+  c.n0 = (t / tm) * p.bn;
   c.w_row0 = c.m0;
   c.row_end = p.rows;
-  c.out_off = 0;
   return c;
 }
 
@@ -85,7 +93,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   sm100::tc_fence_after_sync();
 
   const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
-  const int tiles_total = (p.n_out + 2 * kTileM - 1) / (2 * kTileM) * ((p.rows + p.bn - 1) / p.bn);
+  // (a table is written by the kernels before this one: its length is read behind the wait)
+  auto tile_count = [&] { return p.tile_table != nullptr ? *p.n_tiles / 2 : (p.n_out + 2 * kTileM - 1) / (2 * kTileM) * ((p.rows + p.bn - 1) / p.bn); };
   const uint32_t tiles_addr = sm100::smem_u32(tiles);
   const uint32_t full0 = sm100::smem_u32(&bar->full[0]), empty0 = sm100::smem_u32(&bar->empty[0]);
   const uint32_t stages = static_cast<uint32_t>(L.stages);
@@ -108,13 +117,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         sm100::tma_load_2d_pair(tiles_addr + stage * L.stage_bytes + L.a_bytes, tx, full_even + stage * 8, kb * kTileK, c.n0 + rank * (p.bn / 2), pol_x);
     };
     int early = 0;
-    if (p.w_static && pair < tiles_total) {
+    if (p.w_static && p.tile_table == nullptr && pair < tile_count()) {
       const TileCoord c = pair_coord(p, pair, rank);
       early = min(c.kbn, L.stages);
       for (int i = 0; i < early; ++i) load_w(c, i, i);
     }
     pdl::wait();
     pdl::release();
+    const int tiles_total = tile_count();
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     for (int t = pair; ok && t < tiles_total; t += pairs) {
@@ -137,6 +147,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   } else if (warp == 1) {
     pdl::wait();
     pdl::release();
+    const int tiles_total = tile_count();
     if (rank == 0) {
       const bool leader = sm100::elect_one();
       const uint32_t idesc = sm100::umma_idesc_bf16(2 * kTileM, static_cast<uint32_t>(p.bn));
@@ -177,6 +188,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   } else {
     pdl::wait();
     pdl::release();
+    const int tiles_total = tile_count();
     const int ew = warp & 3, half = (warp - 2) >> 2;
     const uint32_t empty_even = sm100::map_rank(sm100::smem_u32(&bar->acc_empty[0]), 0);
     uint32_t acc = 0, acc_phase = 0;
@@ -190,7 +202,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       sm100::tc_fence_after_sync();
       const uint32_t tmem_acc = bar->tmem_base + acc * acc_cols + (static_cast<uint32_t>(ew * 32) << 16);
       const int f = c.m0 + ew * 32 + lane, cols = min(p.bn, c.row_end - c.n0);
-      epilogue_columns<kWide>(p, c, f, f, tmem_acc, half * (p.bn / 2), min(cols, (half + 1) * (p.bn / 2)), stores_wide<kWide>(p, c.m0 + ew * 32));
+      epilogue_columns<kWide>(p, c, f, c.w_row0 + ew * 32 + lane, tmem_acc, half * (p.bn / 2), min(cols, (half + 1) * (p.bn / 2)), stores_wide<kWide>(p, c.m0 + ew * 32));
       sm100::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive_cluster(empty_even + acc * 8);
@@ -246,14 +258,19 @@ static int resident_pairs(int dev, int sms) {
 // so pairs take a call whose tiles, counted by the rows in them, fill 0.6 of the SMs: with fewer the single-CTA kernel cuts finer.
 // Callers that name a tile width, a split or an SM count mean that kernel.
 int pair_width(const XpGemmArgs& a, int sms) {
-  if (a.fp8 || a.w_tiled || a.tile_table != nullptr || a.batch > 1 || a.splits > 0 || a.bn > 0 || a.num_sms > 0 || a.smem_limit > 0 || a.rows <= 256)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (a.tile_table != nullptr) {     // grouped: where a group's rows fill the wide tiles that the caller chose
+    const bool fits = a.tile_pairs && a.n_out % (2 * kTileM) == 0 && (a.bn == 128 || a.bn == 256) && a.splits <= 1 && a.num_sms == 0 &&
+                      a.smem_limit == 0 && !a.fp8 && !a.w_tiled;
+    return fits && resident_pairs(dev, sms) > 0 ? a.bn : 0;
+  }
+  if (a.fp8 || a.w_tiled || a.batch > 1 || a.splits > 0 || a.bn > 0 || a.num_sms > 0 || a.smem_limit > 0 || a.rows <= 256)
     return 0;
   auto filled = [&](int width) { return static_cast<double>(a.rows) / ((a.rows + width - 1) / width * width); };
   const int width = a.dual && (a.k < 2048 || filled(256) < 0.7) ? 128 : 256;
   const int tiles = (a.n_out + 2 * kTileM - 1) / (2 * kTileM) * ((a.rows + width - 1) / width);
   if (tiles * filled(width) < 0.6 * (sms / 2)) return 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
   return resident_pairs(dev, sms) > 0 ? width : 0;
 }
 
@@ -265,7 +282,7 @@ int pair_launch(const XpGemmArgs& a, Problem p, const CUtensorMap& tmap_w, int w
   if (tmap::cache().get(&tx, a.x, a.rows, a.k, static_cast<uint64_t>(a.ldx > 0 ? a.ldx : a.k) * 2, width / 2, 2) != 0) return -21;
   p.bn = width;
   p.splits = 1;
-  const int tiles = (p.n_out + 2 * kTileM - 1) / (2 * kTileM) * ((p.rows + width - 1) / width);
+  const int tiles = p.tile_table != nullptr ? resident : (p.n_out + 2 * kTileM - 1) / (2 * kTileM) * ((p.rows + width - 1) / width);
   const int nacc = width * (p.dual ? 2 : 1) * 2 <= 512 ? 2 : 1;
   const cudaError_t e = pdl::launch(wide_epilogue ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, 2 * std::min(resident, tiles), kPThreads,
                                     pair_layout(width, p.dual).total_bytes, reinterpret_cast<cudaStream_t>(a.stream), 2, tmap_w, tx, p, nacc, a.status);

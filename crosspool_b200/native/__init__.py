@@ -74,6 +74,7 @@ class GemmArgs(C.Structure):
         ("ld_tail", C.c_int),
         ("relu2", C.c_int),
         ("w_static", C.c_int),
+        ("tile_pairs", C.c_int),
     ]
 
 

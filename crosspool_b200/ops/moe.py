@@ -45,6 +45,8 @@ class MoeWorkspace:
     logits32: torch.Tensor | None = None   # fp32 router logits, allocated on first use by an fp32 router projection
 
 
+ONE_LAUNCH_ROWS, ONE_LAUNCH_EXPERTS = 128, 256      # what xp_moe_topk_route takes: one CTA does it all
+
 ROUTER_PRECISIONS = {"payload": 0, "fp32_logits": 1, "fp32": 2}
 
 
@@ -152,6 +154,7 @@ def _grouped(x, w2d, out, *, n_out, rows_cap, bn, dual, up_offset, tiles, n_tile
     a = gemm._args(x, w2d, out, n_out=n_out, rows=rows_cap, epilogue=epilogue, dual=dual, up_offset=up_offset, splits=1, bn=bn,
                    bias=bias, gate_limit=transform[0], up_add=transform[1], act_alpha=transform[2])
     a.relu2 = relu2
+    a.tile_pairs = int(n_out % 256 == 0)      # the route kernels put the feature tiles of a row tile side by side
     a.tile_table, a.n_tiles, a.w_rows_per_group = tiles.data_ptr(), n_tiles.data_ptr(), rows_per_group
     native.check(native.kernels().xp_gemm(C.byref(a)), "xp_gemm(grouped)")
 
@@ -190,14 +193,18 @@ def moe_forward(x: torch.Tensor, w: FfnLayerWeights, cfg: ModelConfig, out: torc
         if ws.logits32 is None:
             ws.logits32 = torch.zeros(ws.cap_rows, ws.logits.shape[1], dtype=torch.float32, device=dev)
         logits = router_project_fp32(x, w, ws.logits32[:rows])
-    router_topk(logits, e_total, k, out_ids=ws.ids[:rows], out_weights=ws.weights[:rows],
-                sigmoid=cfg.router_scoring == "sigmoid", renormalize=cfg.norm_topk_prob, scale=cfg.routed_scaling_factor,
-                correction_bias=w.extra.get("correction_bias"), logit_bias=w.extra.get("router_bias"),
-                round_weights_bf16=bool(w.extra.get("round_topk_weights")))
-    # 2. order the routes of the local experts, build the tile tables
+    a = _router_args(logits, e_total, k, ws.ids[:rows], ws.weights[:rows], sigmoid=cfg.router_scoring == "sigmoid",
+                     renormalize=cfg.norm_topk_prob, scale=cfg.routed_scaling_factor, correction_bias=w.extra.get("correction_bias"),
+                     logit_bias=w.extra.get("router_bias"), round_weights_bf16=bool(w.extra.get("round_topk_weights")))
+    # 2. order the routes of the local experts, build the tile tables: with few rows in the launch that chooses the experts
+    #    (24 rows of 128 experts: five launches, 18.6 us -> one, 15.9 us)
     bn = _tile_width(rows, k, n_local)
     r = _route_args(ws, rows, k, lo, hi, inter, h, bn)
-    native.check(lib.xp_moe_route(C.byref(r), s), "xp_moe_route", 3)
+    if rows <= ONE_LAUNCH_ROWS and n_local <= ONE_LAUNCH_EXPERTS:
+        native.check(lib.xp_moe_topk_route(C.byref(a), C.byref(r), s), "xp_moe_topk_route")
+    else:
+        native.check(lib.xp_router_topk(C.byref(a), s), "xp_router_topk")
+        native.check(lib.xp_moe_route(C.byref(r), s), "xp_moe_route", 3)
     # 3. gather rows into expert order
     routes = rows * k
     native.check(lib.xp_moe_gather(x.data_ptr(), ws.perm_token.data_ptr(), ws.offsets.data_ptr() + 4 * n_local,
@@ -311,7 +318,7 @@ def routed_ffn(x: torch.Tensor, w: FfnLayerWeights, spec: MoeSpec, out: torch.Te
     a.always = int(fold)
     r = _route_args(ws, rows, k, 0, E, n_gu, h, bn)
     r.bn_gateup = bn_gu
-    if rows <= 128:
+    if rows <= ONE_LAUNCH_ROWS:
         native.check(lib.xp_moe_topk_route(C.byref(a), C.byref(r), s), "xp_moe_topk_route")
     else:
         native.check(lib.xp_router_topk(C.byref(a), s), "xp_router_topk")
