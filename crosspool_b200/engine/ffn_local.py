@@ -15,7 +15,7 @@ from ..models.config import ModelConfig
 from ..models.layered import ceil8, pad_pitch
 from ..models.weights import FfnLayerWeights
 from ..ops import gemm
-from .atn_engine import FfnPort
+from .atn_engine import FfnPort, alike
 
 
 class LocalFfnPort(FfnPort):
@@ -82,6 +82,22 @@ class LocalFfnPort(FfnPort):
             gemm.gateup_swiglu(x, w.gate_up, out=act, gate_limit=limit, up_add=up_add, act_alpha=alpha, act_cubic=cubic, w_static=True)
         gemm.linear(act, w.down, out=self.y[:rows], w_static=True)
         return [self.y[:rows]]
+
+    def plain_layers(self, x: torch.Tensor, rows: int):
+        """(gate/up arguments, down arguments, output) of layer 0, if every layer is a plain bf16 FFN of the same shape that ``run`` would
+        give the same arguments but for the weights; otherwise None."""
+        f0 = self.weights[0] if self.weights else None
+        if type(self).run is not LocalFfnPort.run or f0 is None or f0.is_moe or self.cfg.layered:
+            return None
+        for f in self.weights:
+            if (f is None or f.is_moe or f.extra or not alike(f.gate_up, f0.gate_up) or not alike(f.down, f0.down)
+                    or not alike(f.gate_up_bias, f0.gate_up_bias) or not alike(f.down_bias, f0.down_bias)):
+                return None
+        inter, n, y = f0.gate_up.shape[0] // 2, f0.down.shape[0], self.y[:rows]
+        act = self.act[:rows, :inter]
+        gu = gemm._args(x, f0.gate_up, act, n_out=inter, rows=rows, epilogue=gemm.EPI_SWIGLU, dual=1, up_offset=inter, bias=f0.gate_up_bias, w_static=True)
+        dn = gemm._args(act, f0.down, y, n_out=n, rows=rows, epilogue=gemm.EPI_STORE, bias=f0.down_bias, w_static=True)
+        return gu, dn, y
 
     def run(self, layer: int, x: torch.Tensor, rows: int, mode: int) -> list[torch.Tensor]:
         w = self.weights[layer]

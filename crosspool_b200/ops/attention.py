@@ -24,6 +24,11 @@ def rope_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor,
                   theta: float, q_norm: torch.Tensor | None = None, k_norm: torch.Tensor | None = None,
                   eps: float = 1e-6) -> None:
     """qkv ``[rows, (q+2kv)*d]`` → RoPE'd q in ``q_out`` and k/v scattered to the paged cache."""
+    a = rope_args(qkv, q_out, k_cache, v_cache, positions, slots, q_heads, kv_heads, head_dim, theta, q_norm, k_norm, eps)
+    native.check(native.kernels().xp_rope_kv(C.byref(a), _stream(qkv.device)), "xp_rope_kv")
+
+
+def rope_args(qkv, q_out, k_cache, v_cache, positions, slots, q_heads, kv_heads, head_dim, theta, q_norm, k_norm, eps) -> "native.RopeArgs":
     a = native.RopeArgs()
     a.qkv, a.q_out = qkv.data_ptr(), q_out.data_ptr()
     a.k_cache, a.v_cache = k_cache.data_ptr(), v_cache.data_ptr()
@@ -34,7 +39,7 @@ def rope_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor,
     a.rows, a.ld_qkv = qkv.shape[0], qkv.stride(0)
     a.q_heads, a.kv_heads, a.head_dim = q_heads, kv_heads, head_dim
     a.eps, a.log2_theta = eps, math.log2(theta)
-    native.check(native.kernels().xp_rope_kv(C.byref(a), _stream(qkv.device)), "xp_rope_kv")
+    return a
 
 
 def decode_splits(batch: int, kv_heads: int, max_len: int) -> int:
@@ -118,10 +123,16 @@ def paged_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
     Runs the tcgen05 kernel (S and O in tensor memory, TMA-fed Q/K/V, the heads of a KV group packed into 128-row
     tiles) when pages hold a power-of-two number of at least 16 tokens and 1, 2, 4, 8 or 16 query heads share a KV
     head. ``force_simple``: True or ``"simple"`` selects the plain kernel, ``"mma"`` the TMA-fed mma.sync kernel."""
-    _, q_heads, d = q.shape
-    page_size, kv_heads = k_cache.shape[1], k_cache.shape[2]
     if out is None:
         out = torch.empty_like(q)
+    a = prefill_args(q, k_cache, v_cache, block_table, q_starts, q_lens, ctx_lens, max_q_len, out, scale, force_simple)
+    native.check(native.kernels().xp_prefill_attn(C.byref(a), _stream(q.device)), "xp_prefill_attn")
+    return out
+
+
+def prefill_args(q, k_cache, v_cache, block_table, q_starts, q_lens, ctx_lens, max_q_len, out, scale=None, force_simple=None) -> "native.PrefillAttnArgs":
+    _, q_heads, d = q.shape
+    page_size, kv_heads = k_cache.shape[1], k_cache.shape[2]
     a = native.PrefillAttnArgs()
     a.q, a.k_cache, a.v_cache, a.out = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr()
     a.block_table = block_table.data_ptr()
@@ -137,8 +148,7 @@ def paged_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
     from .gemm import status_words
 
     a.status = status_words(q.device).data_ptr()
-    native.check(native.kernels().xp_prefill_attn(C.byref(a), _stream(q.device)), "xp_prefill_attn")
-    return out
+    return a
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:

@@ -29,6 +29,16 @@ def _done_counter(device: torch.device) -> torch.Tensor:
     return t
 
 
+def local_args(part: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor, resid: torch.Tensor | None = None) -> native.NormArgs:
+    """Arguments of one norm of local rows with model weights, for callers that issue ``xp_norm_publish`` layer by layer."""
+    a = native.NormArgs()
+    a.parts[0], a.weight, a.out_local = part.data_ptr(), weight.data_ptr(), out.data_ptr()
+    a.resid = resid.data_ptr() if resid is not None else None
+    a.rows, a.hidden = part.shape
+    a.ld_parts, a.ld_out, a.nparts, a.eps, a.w_static = part.stride(0), out.stride(0), 1, eps, 1
+    return a
+
+
 def add_rmsnorm(parts: Sequence[torch.Tensor] | torch.Tensor, weight: torch.Tensor | None, eps: float = 1e-6, *,
                 resid: torch.Tensor | None = None, out: torch.Tensor | None = None,
                 peer_ptrs: Sequence[int] = (), peer_flag_ptrs: Sequence[int] = (), peer_meta_ptrs: Sequence[int] = (),
