@@ -1,0 +1,59 @@
+"""Edges of the row kernels: rows of a warp and of a CTA, rows in several CTAs' heads, rows off 4- and 16-byte boundaries, whole clusters."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("static", [False, True])
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (9, 1016), (7, 1024), (8, 1032), (3, 8192)])
+def test_norm_rows(rows, hidden, static):
+    from crosspool_b200.ops import norm
+
+    g = torch.Generator(device="cuda").manual_seed(rows + hidden)
+    p, r = (torch.randn(rows, hidden, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda", generator=g)).bfloat16()
+    torch.cuda.synchronize()
+    s = (p.float() + r.float()).bfloat16()
+    want = (s.float() * torch.rsqrt(s.float().square().mean(-1, keepdim=True) + 1e-6)).bfloat16().float() * w.float()
+    y = norm.add_rmsnorm([p], w, 1e-6, resid=r, w_static=static)
+    assert torch.equal(r, s)
+    torch.testing.assert_close(y.float(), want, rtol=2.0 ** -7, atol=1e-6)      # two roundings to bf16
+
+
+@pytest.mark.parametrize("rows", [591, 592])          # a warp per head; a CTA per row
+@pytest.mark.parametrize("pad", [0, 1])               # odd pitches: no 4-byte loads
+def test_rope_rows(rows, pad):
+    from crosspool_b200.ops import attention as A
+
+    hq, hk, d = 5, 3, 128
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    qkv = torch.randn(rows, (hq + 2 * hk) * d + pad, device="cuda", generator=g).bfloat16()[:, :(hq + 2 * hk) * d]
+    q = torch.empty(rows, hq, d, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.zeros(rows // 16 + 1, 16, hk, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    pos = torch.arange(rows, device="cuda", dtype=torch.int32)
+    slots = pos.clone()
+    slots[5] = -1
+    A.rope_kv_write(qkv, q, k, v, pos, slots, q_heads=hq, kv_heads=hk, head_dim=d, theta=1e4)
+    x = qkv.float().view(rows, hq + 2 * hk, d) if not pad else qkv.float().reshape(rows, hq + 2 * hk, d)
+    f = 1e4 ** (-torch.arange(0, d, 2, device="cuda").double() / d)
+    c, s = (t[:, None] for t in ((pos[:, None] * f).cos().float(), (pos[:, None] * f).sin().float()))
+    a, b = x[..., :d // 2], x[..., d // 2:]
+    rot = torch.cat([a * c - b * s, b * c + a * s], -1)
+    keep = slots >= 0
+    # angles are fp32: at position p they are off by p 2^-23 or so, which turns a pair by as much
+    torch.testing.assert_close(q.float(), rot[:, :hq], rtol=2.0 ** -8, atol=2e-3)
+    torch.testing.assert_close(k.view(-1, hk, d)[:rows][keep].float(), rot[keep][:, hq:hq + hk], rtol=2.0 ** -8, atol=2e-3)
+    assert torch.equal(v.view(-1, hk, d)[:rows][keep].float(), x[keep][:, hq + hk:]) and not k.view(-1, hk, d)[5].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab", [1, 7, 8, 2049, 151936])
+def test_argmax_rows(vocab, dtype):
+    from crosspool_b200.ops import attention as A
+
+    x = torch.randn(9, vocab, device="cuda", generator=torch.Generator(device="cuda").manual_seed(vocab)).to(dtype)
+    x[1] = -float("inf")
+    x[2, vocab // 2] = x[2, vocab - 1] = float("inf")      # ties go to the lower id
+    want = torch.stack([(r == r.max()).nonzero()[0, 0] for r in x]).int()
+    assert torch.equal(A.argmax(x), want)
