@@ -3,6 +3,8 @@
 #include <cooperative_groups.h>
 #include <math_constants.h>
 
+#include <utility>
+
 #include "xpool/api.h"
 #include "xpool/pdl.cuh"
 #include "xpool/sm100.cuh"
@@ -48,6 +50,9 @@ template <typename T>
 __global__ void __launch_bounds__(kArgThreads)
 argmax_kernel(const T* logits, int* out, int vocab, int ld, int wide) {
   namespace cg = cooperative_groups;
+  // The first CTA's shared memory may be written once that CTA is known to have started: all arrive here and wait before the
+  // stores, a row's scan later.
+  auto started = cg::this_cluster().barrier_arrive();
   xpool::pdl::wait();
   xpool::pdl::release();
   constexpr int N = 16 / sizeof(T), kWarps = kArgThreads / 32;
@@ -68,6 +73,7 @@ argmax_kernel(const T* logits, int* out, int vocab, int ld, int wide) {
   }
   for (int i = whole * N + first; i < vocab; i += kStride) better(best, bi, to_f<T>(row[i]), i);
   warp_best(best, bi);
+  cg::this_cluster().barrier_wait(std::move(started));
   if ((threadIdx.x & 31) == 0) {
     const int slot = rank * kWarps + (threadIdx.x >> 5);
     cg::this_cluster().map_shared_rank(sv, 0)[slot] = best;

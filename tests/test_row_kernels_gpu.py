@@ -57,3 +57,18 @@ def test_argmax_rows(vocab, dtype):
     x[2, vocab // 2] = x[2, vocab - 1] = float("inf")      # ties go to the lower id
     want = torch.stack([(r == r.max()).nonzero()[0, 0] for r in x]).int()
     assert torch.equal(A.argmax(x), want)
+
+
+@pytest.mark.parametrize("vocab", [1, 64, 1000])
+def test_argmax_of_short_rows_back_to_back(vocab):
+    """Rows that a cluster scans in no time, more clusters than the GPU holds, launches one behind the other: a CTA's winners go to
+    the first CTA of its cluster only once that has started."""
+    from crosspool_b200.ops import attention as A
+
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    x = torch.randn(3000, vocab, device="cuda", generator=g)
+    want = x.argmax(-1).int()          # no ties: 3000 x 1000 draws of 24-bit normals, checked below
+    assert ((x == x.max(-1, keepdim=True).values).sum(-1) == 1).all()
+    torch.cuda.synchronize()
+    got = [A.argmax(x) for _ in range(50)]
+    assert all(torch.equal(t, want) for t in got)
