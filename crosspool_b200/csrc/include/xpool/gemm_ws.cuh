@@ -686,11 +686,11 @@ __device__ __forceinline__ bool epilogue_tile(const Problem& p, const TileCoord&
     for (int i = 0; i < c.kbn; ++i) {
       // The scales of this K block do not depend on its MMAs: their loads are issued before the wait
       // for the accumulator so that the L2 round trip overlaps it.
-      const float sw = __ldg(wsc + i);
+      const float sw = wsc[i];
       const float4* xs = reinterpret_cast<const float4*>(p.x_scale + static_cast<size_t>(c.kb0 + i) * p.ld_xscale + c.n0);
       float4 sx[kMaxBnF8 / 4];
 #pragma unroll
-      for (int q = 0; q < kMaxBnF8 / 4; ++q) sx[q] = q * 4 < p.bn ? __ldg(xs + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int q = 0; q < kMaxBnF8 / 4; ++q) sx[q] = q * 4 < p.bn ? xs[q] : make_float4(0.f, 0.f, 0.f, 0.f);
       if (i > 0) {
         if (!__all_sync(0xffffffffu, sm100::mbar_wait(&bar->acc_full[st.acc], st.acc_phase, deadline))) return false;
         sm100::tc_fence_after_sync();

@@ -533,7 +533,7 @@ prefill_attn_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                                   (stored ? hq : 0) * a.v_valid;
 #pragma unroll
         for (int i = 0; i < DV / 8; ++i)
-          asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
+          asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(gate_row[i].x), "=r"(gate_row[i].y), "=r"(gate_row[i].z), "=r"(gate_row[i].w)
                        : "l"(ge + min(i * 8, a.v_valid - 8)));
       }

@@ -37,9 +37,10 @@ struct StreamArgs {
   Problem p;
 };
 
+// (a coherent load: where w_static is 0 the previous kernel may still write w after this one has begun)
 __device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 
