@@ -156,12 +156,11 @@ norm_rows_kernel(XpNormArgs a) {
   }
 }
 
-// General form: one CTA per row; hidden % 8 == 0; hidden <= 8 * kThreads * kMaxVec.
+// General form: one CTA per row; hidden % 8 == 0; hidden <= 8 * kThreads * kMaxVec. An ordinary launch, on both sides: CTAs that are
+// resident early would take the room of the kernels whose flags they spin on.
 
 __global__ void __launch_bounds__(kThreads)
 norm_publish_kernel(XpNormArgs a) {
-  // A CTA that may spin on another GPU's flag holds its successor back: CTAs resident early would take the room of what it waits for.
-  pdl::wait();
   __shared__ float red[kThreads / 32];
   __shared__ uint32_t s_fail;
   const int row = blockIdx.x;
@@ -331,7 +330,7 @@ extern "C" int xp_norm_publish(const XpNormArgs* a, void* stream) {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
   }
-  xpool::pdl::launch(xpool::norm::norm_publish_kernel, a->rows, xpool::norm::kThreads, 0, reinterpret_cast<cudaStream_t>(stream), 1, *a);
+  xpool::norm::norm_publish_kernel<<<a->rows, xpool::norm::kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }

@@ -107,3 +107,9 @@ def test_early_kernels_wait_before_they_let_the_next_one_start(source, kernel):
     for body in bodies:
         wait, release = _first(r"pdl::wait\(\)", body), _first(r"pdl::release\(\)", body)
         assert wait is not None and (release is None or wait < release), kernel
+
+
+@pytest.mark.parametrize("source,kernel", DEPENDENT)
+def test_kernels_that_handshake_with_other_gpus_do_not_start_early(source, kernel):
+    for name, body in _reached(source, kernel).items():
+        assert re.search(r"\b(wait_flag_ge|st_release_sys|ld_acquire_sys)\(", body) is None, f"{kernel}: {name}"
