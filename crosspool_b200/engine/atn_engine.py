@@ -390,7 +390,8 @@ class AttentionEngine:
         cfg, layers, kv = self.cfg, self.w.layers, self.kv
         l0, plain = layers[0], getattr(self.port, "plain_layers", None)
         resid, x, x2, o = self.resid[:rows], self.x[:rows], self.x2[:rows], self.o[:rows]
-        if self.tp is not None or plain is None or not isinstance(l0.qkv, torch.Tensor) or not isinstance(l0.o, torch.Tensor):
+        if (self.tp is not None or plain is None or len(self.port.weights) < len(layers) or not isinstance(l0.qkv, torch.Tensor)
+                or not isinstance(l0.o, torch.Tensor)):
             return False
         for l, lw in enumerate(layers):
             if not (alike(lw.qkv, l0.qkv) and alike(lw.o, l0.o) and alike(lw.qkv_bias, l0.qkv_bias) and alike(lw.q_norm, l0.q_norm)

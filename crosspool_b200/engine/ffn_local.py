@@ -85,9 +85,10 @@ class LocalFfnPort(FfnPort):
 
     def plain_layers(self, x: torch.Tensor, rows: int):
         """(gate/up arguments, down arguments, output) of layer 0, if every layer is a plain bf16 FFN of the same shape that ``run`` would
-        give the same arguments but for the weights; otherwise None."""
+        give the same arguments but for the weights; otherwise None, also where a subclass, an instance or a patched class answers for a
+        layer in another way."""
         f0 = self.weights[0] if self.weights else None
-        if type(self).run is not LocalFfnPort.run or f0 is None or f0.is_moe or self.cfg.layered:
+        if any(n in vars(self) or getattr(type(self), n) is not f for n, f in _ASKED.items()) or f0 is None or f0.is_moe or self.cfg.layered:
             return None
         for f in self.weights:
             if (f is None or f.is_moe or f.extra or not alike(f.gate_up, f0.gate_up) or not alike(f.down, f0.down)
@@ -121,6 +122,10 @@ class LocalFfnPort(FfnPort):
         gemm.gateup_swiglu(x, w.gate_up, out=act, bias=w.gate_up_bias, gate_limit=lim, up_add=up_add, act_alpha=alpha, w_static=True)
         gemm.linear(act, w.down, out=self.y[:rows], bias=w.down_bias, w_static=True)
         return [self.y[:rows]]
+
+
+# what a layer asks of a port
+_ASKED = {n: getattr(LocalFfnPort, n) for n in ("run", "publish_targets", "wait_args")}
 
 
 class UnfusedFfnPort(FfnPort):
