@@ -378,11 +378,12 @@ class AttentionEngine:
             parts = self.port.run(l, x2, rows, mode)
         self._parts = parts
 
-    def _plain_layers(self, rows: int, rope, att) -> bool:
+    def _plain_layers(self, rows: int, attn_args) -> bool:
         """The layers of a prefill pass over local weights of one shape: the launches of ``_layers``, with every kernel's arguments
         built once a pass and only the layer's addresses set per layer. (Built anew for every launch they took 18 us of host time
-        each, 4.2 ms for the 228 launches of a 28-layer model, whose kernels run 2 ms over a short prompt.) ``rope`` and ``att``: the
-        arguments of layer 0. Returns False, with nothing launched, where the layers are not like that."""
+        each, 4.2 ms for the 228 launches of a 28-layer model, whose kernels run 2 ms over a short prompt.) ``attn_args`` gives the
+        rotation's and the attention's arguments of layer 0. Returns False, with nothing launched, where the layers are not like that;
+        the port is asked first, because it knows at once (routed layers, FFNs elsewhere)."""
         import ctypes as C
 
         from .. import native
@@ -393,14 +394,15 @@ class AttentionEngine:
         if (self.tp is not None or plain is None or len(self.port.weights) < len(layers) or not isinstance(l0.qkv, torch.Tensor)
                 or not isinstance(l0.o, torch.Tensor)):
             return False
+        ffn = plain(x2, rows)
+        if ffn is None:
+            return False
         for l, lw in enumerate(layers):
             if not (alike(lw.qkv, l0.qkv) and alike(lw.o, l0.o) and alike(lw.qkv_bias, l0.qkv_bias) and alike(lw.q_norm, l0.q_norm)
                     and alike(lw.k_norm, l0.k_norm) and alike(lw.input_norm, l0.input_norm) and alike(lw.post_attn_norm, l0.input_norm)
                     and alike(kv.k[l], kv.k[0]) and alike(kv.v[l], kv.v[0])):
                 return False
-        ffn = plain(x2, rows)
-        if ffn is None:
-            return False
+        rope, att = attn_args()
         gu, dn, y = ffn
         qkv = gemm._args(x, l0.qkv, self.qkv[:rows], n_out=l0.qkv.shape[0], rows=rows, epilogue=gemm.EPI_STORE, bias=l0.qkv_bias, w_static=True)
         proj = gemm._args(self.attn_out[:rows].view(rows, cfg.q_size), l0.o, o, n_out=l0.o.shape[0], rows=rows, epilogue=gemm.EPI_STORE, w_static=True)
@@ -492,11 +494,13 @@ class AttentionEngine:
             A.paged_prefill(self.q[:r], self.kv.k[l], self.kv.v[l], table, q_starts, q_lens, ctx_lens, max_q,
                             out=self.attn_out[:r])
 
-        l0 = self.w.layers[0]
-        rope = A.rope_args(self.qkv[:rows], self.q[:rows], self.kv.k[0], self.kv.v[0], pos, slots, cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim,
-                           cfg.rope_theta, l0.q_norm, l0.k_norm, cfg.rms_norm_eps)
-        att = A.prefill_args(self.q[:rows], self.kv.k[0], self.kv.v[0], table, q_starts, q_lens, ctx_lens, max_q, self.attn_out[:rows])
-        if not self._plain_layers(rows, rope, att):
+        def attn_args():
+            l0 = self.w.layers[0]
+            rope = A.rope_args(self.qkv[:rows], self.q[:rows], self.kv.k[0], self.kv.v[0], pos, slots, cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim,
+                               cfg.rope_theta, l0.q_norm, l0.k_norm, cfg.rms_norm_eps)
+            return rope, A.prefill_args(self.q[:rows], self.kv.k[0], self.kv.v[0], table, q_starts, q_lens, ctx_lens, max_q, self.attn_out[:rows])
+
+        if not self._plain_layers(rows, attn_args):
             self._layers(rows, MODE_PREFILL, attn)
         self._head(rows, n_seqs, last_idx)
 

@@ -133,3 +133,20 @@ def test_overridden_ports_see_every_layer(kind, monkeypatch):
     e = _engine(port=lambda cfg, fw: _overridden(kind, _port()[0], cfg, fw, calls, monkeypatch))
     _first_logits(e)
     assert len(calls) == 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("preset,change,built,compared", [("Qwen/Qwen3-0.6B", None, 1, True), ("Qwen/Qwen3-0.6B", _biased, 3, False),
+                                                          ("Qwen/Qwen3-30B-A3B", None, 3, False)])
+def test_refused_passes_pay_for_no_arguments_of_their_own(preset, change, built, compared, monkeypatch):
+    """Launch arguments are built once where the layers are plain and once a layer where the port says at once that they are not,
+    without a look at the attention's weights."""
+    from crosspool_b200.engine import atn_engine
+    from crosspool_b200.ops import attention as A
+
+    e, seen, looks = _engine(preset, change=change), [], []
+    args, alike = A.rope_args, atn_engine.alike
+    monkeypatch.setattr(A, "rope_args", lambda *a: seen.append(1) or args(*a))
+    monkeypatch.setattr(atn_engine, "alike", lambda a, b: looks.append(1) or alike(a, b))
+    _first_logits(e)
+    assert len(seen) == built and bool(looks) == compared
