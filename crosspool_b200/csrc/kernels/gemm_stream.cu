@@ -222,8 +222,12 @@ gemm_stream_kernel(const __grid_constant__ StreamArgs a) {
 //   gate/up 24576 x 4096   42.5 -> 36.7    42.2 -> 38.1    42.1 -> 41.8    41.4 -> 73.6
 //   4096 x 12288           29.7 -> 17.8    29.6 -> 18.4    29.7 -> 20.7    31.1 -> 33.8
 // From two eights on a warp takes 32 features, which halves what it reads of the activations. Calls that name a tile width,
-// a split or an SM count mean the tiled kernel; rows of K that are no whole 16-byte units need its zero-filled tiles.
+// a split or an SM count mean the tiled kernel; rows of K that are no whole 16-byte units, and features whose weight rows the caller
+// says do not exist (w_rows_total), need its zero-filled tiles.
 bool stream_applies(const XpGemmArgs& a) {
+  const int groups = a.batch > 1 ? a.batch - 1 : 0;
+  const int64_t w_rows = a.n_out + static_cast<int64_t>(groups) * a.w_rows_per_group + (a.dual ? a.up_offset : 0);
+  if (a.w_rows_total > 0 && (a.w_rows_total < w_rows || (a.w_tiled && a.w_rows_total % kTileM != 0))) return false;
   const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return a.rows <= kStreamMaxRows && !a.fp8 && a.tile_table == nullptr && a.splits == 0 && a.bn == 0 && a.num_sms == 0 && a.k % 8 == 0 &&
          (a.ldw == 0 || a.ldw % 8 == 0) && (a.ldx == 0 || a.ldx % 8 == 0) && aligned(a.w) && aligned(a.x) &&

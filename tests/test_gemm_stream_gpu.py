@@ -95,3 +95,33 @@ def test_refuses_what_it_refused():
         gemm.linear(flat[1:].view(4, 64), w)
     with pytest.raises(native.NativeLibraryError):
         gemm.linear(torch.zeros(4, 68, device="cuda", dtype=torch.bfloat16)[:, :64], w)
+
+
+def _raw(x, w, n_out, w_rows_total, **kw):
+    import ctypes as C
+
+    from crosspool_b200 import native
+    from crosspool_b200.ops import gemm
+
+    out = torch.full((x.shape[0], n_out), 7.0, device="cuda", dtype=torch.bfloat16)
+    a = gemm._args(x, w, out, n_out=n_out, rows=x.shape[0], epilogue=kw.pop("epilogue", gemm.EPI_STORE), **kw)
+    a.w_rows_total = w_rows_total
+    native.check(native.kernels().xp_gemm(C.byref(a)), "xp_gemm")
+    return out
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17])     # 17: the tiled kernel
+def test_features_without_weight_rows_are_zero(rows):
+    """A caller that names fewer weight rows than features gets zeros there, whichever kernel runs; nothing is read behind them."""
+    from crosspool_b200 import native
+    from crosspool_b200.ops import gemm
+
+    x, w, _ = _data(rows, 200, 256, rows)
+    want = x.float() @ w.float().t()
+    want[:, 130:] = 0
+    _close(_raw(x, w, 200, 130), want)
+    gate, up = want[:, :100].bfloat16().float(), want[:, 100:].bfloat16().float()
+    _close(_raw(x, w, 100, 130, epilogue=gemm.EPI_SWIGLU, dual=1, up_offset=100), torch.nn.functional.silu(gate) * up, 3)
+    tiled = gemm.tile_weight(torch.randn(256, 256, device="cuda").bfloat16())
+    with pytest.raises(native.NativeLibraryError):
+        _raw(x, tiled, 128, 130)
