@@ -711,7 +711,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 template <int D, bool kSig = false, typename A>
 __global__ void decode_combine_kernel(A args, int nsplit) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   const XpDecodeAttnArgs& a = base_of(args);
   const int hq = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const float* ws = a.ws + (static_cast<size_t>(b) * a.q_heads + hq) * nsplit * (D + 2);

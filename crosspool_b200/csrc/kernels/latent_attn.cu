@@ -32,7 +32,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kPrepThreads)
 latent_prep_kernel(XpLatentPrepArgs a) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   extern __shared__ float cs[];            // cos | sin, rot_dims / 2 each
   __shared__ float red[kPrepThreads / 32];
   const int row = blockIdx.x;
@@ -576,7 +576,7 @@ constexpr int kMaxSlices = 64;
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(XpLatentAttnArgs a) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   const int h = blockIdx.x, row = blockIdx.y;
   const bool pad = a.slots[row] < 0;
   const int len = pad ? 0 : a.positions[row] + 1;

@@ -14,7 +14,7 @@ namespace {
 __global__ void __launch_bounds__(128)
 embedding_kernel(const int* ids, const uint4* table, uint4* out, int hidden8, int vocab) {
   xpool::pdl::wait();
-  xpool::pdl::release();
+  xpool::pdl::release_short();
   const int row = blockIdx.x;
   int id = ids[row];
   if (id < 0 || id >= vocab) id = 0;

@@ -128,7 +128,7 @@ __device__ __forceinline__ void router_topk_row(const XpRouterArgs& a, int row, 
 __global__ void __launch_bounds__(128)
 router_topk_kernel(XpRouterArgs a) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= a.rows) return;
   router_topk_row(a, row, threadIdx.x & 31);
@@ -259,7 +259,7 @@ route_place_kernel(const int* ids, int n_routes, int top_k, int lo, const int* o
 __global__ void __launch_bounds__(128)
 gather_rows_kernel(const uint4* x, const int* perm_token, const int* n_rows_ptr, uint4* out, int hidden8, int ldx8) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   const int pos = blockIdx.x;
   if (pos >= *n_rows_ptr) return;
   const uint4* src = x + static_cast<size_t>(perm_token[pos]) * ldx8;
@@ -311,7 +311,7 @@ __device__ __forceinline__ void combine_token(const __nv_bfloat16* y, const int*
 __global__ void __launch_bounds__(128)
 combine_kernel(const __nv_bfloat16* y, const int* route_pos, const float* weights, __nv_bfloat16* out, int top_k, int hidden, int ld_out) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   combine_token(y, route_pos, weights, out, top_k, hidden, ld_out, blockIdx.x, (blockIdx.y * 128 + threadIdx.x) * 8, gridDim.y * 128 * 8);
 }
 

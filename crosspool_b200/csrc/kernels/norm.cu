@@ -74,7 +74,7 @@ norm_rows_kernel(XpNormArgs a) {
   };
   if (a.weight != nullptr && a.w_static) load_weight();
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   if (row >= a.rows) return;     // (whole warps or nobody)
   auto part = [&](int p, int v) {
     return __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.parts[p]) + static_cast<size_t>(row) * a.ld_parts) + v);

@@ -45,7 +45,7 @@ rope_kv_kernel(XpRopeArgs a, int heads_step) {
     }
   };
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   if (first >= heads_total) return;
   const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.qkv) + static_cast<size_t>(row) * a.ld_qkv;
   const __nv_bfloat16* qn = reinterpret_cast<const __nv_bfloat16*>(a.q_norm_weight);

@@ -26,7 +26,7 @@ template <typename T, int N, int KIND>
 __global__ void __launch_bounds__(kThreads)
 resid_norm_kernel(XpResidNormArgs a) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   __shared__ float red[kThreads / 32];
   const int i = blockIdx.x;
   const int r = a.sel != nullptr ? a.sel[i] : i;
@@ -124,7 +124,7 @@ template <typename T, int N>
 __global__ void __launch_bounds__(kThreads)
 polynorm_kernel(XpPolyNormArgs a) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   __shared__ float red[kThreads / 32];
   const T* z = reinterpret_cast<const T*>(a.z) + static_cast<size_t>(blockIdx.x) * a.ld_z;
   T* out = reinterpret_cast<T*>(a.out) + static_cast<size_t>(blockIdx.x) * a.ld_out;
@@ -177,7 +177,7 @@ template <typename T, int N>
 __global__ void __launch_bounds__(kThreads)
 gated_rms_kernel(XpGatedRmsArgs a) {
   pdl::wait();
-  pdl::release();
+  pdl::release_short();
   __shared__ float red[kThreads / 32];
   const float* o = a.o + static_cast<size_t>(blockIdx.x) * a.ld_o;
   const T* gate = reinterpret_cast<const T*>(a.gate) + static_cast<size_t>(blockIdx.x) * a.ld_gate;
