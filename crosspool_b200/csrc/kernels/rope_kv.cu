@@ -13,12 +13,10 @@
 namespace xpool {
 namespace rope {
 
-constexpr int kHeadsInFlight = 4;
-
-// A warp takes every heads_step-th head of a row: the angles are the row's, so their sines are computed once a warp (they were
-// most of the work when every head had a warp of its own), and the loads of four heads are in flight together. Lane l
-// rotates elements l PER .. + PER - 1 of one half with those of the other. WIDE: pairs of elements are 4-byte aligned.
-// 4096 rows of 32 heads of 128: 29.6 -> 26.6 us.
+// A warp takes every heads_step-th head of a row: the angles are the row's, so their sines are computed once a warp. Lane l rotates
+// elements l PER .. + PER - 1 of one half with those of the other. WIDE: pairs of elements are 4-byte aligned. Bound by the latency of a
+// head's loads, so what counts is warps in flight: 32 registers a thread keep every SM full of them. (Four heads of a warp in flight
+// took 64 registers: 4096 rows of 32 query and 8 key heads 47.1 us, so 34.4; 591 rows with a warp a head 10.1 us, so 7.4.)
 template <int D, bool WIDE>
 __global__ void __launch_bounds__(256)
 rope_kv_kernel(XpRopeArgs a, int heads_step) {
@@ -54,70 +52,60 @@ rope_kv_kernel(XpRopeArgs a, int heads_step) {
   const float pos = static_cast<float>(a.positions[row]);
   float c[PER], s[PER];
   bool have = false;
-  for (int h0 = first; h0 < heads_total; h0 += kHeadsInFlight * heads_step) {
-    float x1[kHeadsInFlight][PER], x2[kHeadsInFlight][PER], n1[kHeadsInFlight][PER], n2[kHeadsInFlight][PER];
-#pragma unroll
-    for (int u = 0; u < kHeadsInFlight; ++u) {
-      const int head = h0 + u * heads_step;
-      if (head < heads_total) {
-        load(src + static_cast<size_t>(head) * D, x1[u]);
-        load(src + static_cast<size_t>(head) * D + D / 2, x2[u]);
-        const __nv_bfloat16* nw = head < a.q_heads ? qn : head < rotated ? kn : nullptr;
-        if (nw != nullptr) {
-          load(nw, n1[u]);
-          load(nw + D / 2, n2[u]);
-        }
+  for (int head = first; head < heads_total; head += heads_step) {
+    const bool is_q = head < a.q_heads;
+    float x1[PER], x2[PER];
+    load(src + static_cast<size_t>(head) * D, x1);
+    load(src + static_cast<size_t>(head) * D + D / 2, x2);
+    if (head < rotated) {
+      const __nv_bfloat16* nw = is_q ? qn : kn;
+      float n1[PER], n2[PER];
+      if (nw != nullptr) {
+        load(nw, n1);
+        load(nw + D / 2, n2);
       }
-    }
-    if (!have && h0 < rotated) {      // beside the loads
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const int idx = lane * PER + i;
-        const float inv_freq = exp2f(-(2.f * idx / D) * a.log2_theta);
-        sincosf(pos * inv_freq, &s[i], &c[i]);
-      }
-      have = true;
-    }
-#pragma unroll
-    for (int u = 0; u < kHeadsInFlight; ++u) {
-      const int head = h0 + u * heads_step;
-      if (head >= heads_total) break;
-      const bool is_q = head < a.q_heads;
-      if (head < rotated) {
-        if ((is_q ? qn : kn) != nullptr) {
-          float ss = 0.f;
-#pragma unroll
-          for (int i = 0; i < PER; ++i) ss += x1[u][i] * x1[u][i] + x2[u][i] * x2[u][i];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-          const float inv = rsqrtf(ss / D + a.eps);
-#pragma unroll
-          for (int i = 0; i < PER; ++i) {
-            const float v1 = __bfloat162float(__float2bfloat16_rn(x1[u][i] * inv));
-            const float v2 = __bfloat162float(__float2bfloat16_rn(x2[u][i] * inv));
-            x1[u][i] = __bfloat162float(__float2bfloat16_rn(v1 * n1[u][i]));
-            x2[u][i] = __bfloat162float(__float2bfloat16_rn(v2 * n2[u][i]));
-          }
-        }
+      if (!have) {                      // beside the loads
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
-          const float r1 = x1[u][i] * c[i] - x2[u][i] * s[i];
-          const float r2 = x2[u][i] * c[i] + x1[u][i] * s[i];
-          x1[u][i] = r1;
-          x2[u][i] = r2;
+          const int idx = lane * PER + i;
+          const float inv_freq = exp2f(-(2.f * idx / D) * a.log2_theta);
+          sincosf(pos * inv_freq, &s[i], &c[i]);
+        }
+        have = true;
+      }
+      if (nw != nullptr) {
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) ss += x1[i] * x1[i] + x2[i] * x2[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float inv = rsqrtf(ss / D + a.eps);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          const float v1 = __bfloat162float(__float2bfloat16_rn(x1[i] * inv));
+          const float v2 = __bfloat162float(__float2bfloat16_rn(x2[i] * inv));
+          x1[i] = __bfloat162float(__float2bfloat16_rn(v1 * n1[i]));
+          x2[i] = __bfloat162float(__float2bfloat16_rn(v2 * n2[i]));
         }
       }
-      __nv_bfloat16* dst;
-      if (is_q) {
-        dst = reinterpret_cast<__nv_bfloat16*>(a.q_out) + (static_cast<size_t>(row) * a.q_heads + head) * D;
-      } else {
-        if (slot < 0) continue;
-        const int hk = head < rotated ? head - a.q_heads : head - rotated;
-        dst = reinterpret_cast<__nv_bfloat16*>(head < rotated ? a.k_cache : a.v_cache) + (static_cast<size_t>(slot) * a.kv_heads + hk) * D;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const float r1 = x1[i] * c[i] - x2[i] * s[i];
+        const float r2 = x2[i] * c[i] + x1[i] * s[i];
+        x1[i] = r1;
+        x2[i] = r2;
       }
-      store(dst, x1[u]);
-      store(dst + D / 2, x2[u]);
     }
+    __nv_bfloat16* dst;
+    if (is_q) {
+      dst = reinterpret_cast<__nv_bfloat16*>(a.q_out) + (static_cast<size_t>(row) * a.q_heads + head) * D;
+    } else {
+      if (slot < 0) continue;
+      const int hk = head < rotated ? head - a.q_heads : head - rotated;
+      dst = reinterpret_cast<__nv_bfloat16*>(head < rotated ? a.k_cache : a.v_cache) + (static_cast<size_t>(slot) * a.kv_heads + hk) * D;
+    }
+    store(dst, x1);
+    store(dst + D / 2, x2);
   }
 }
 
@@ -127,7 +115,9 @@ rope_kv_kernel(XpRopeArgs a, int heads_step) {
 extern "C" int xp_rope_kv(const XpRopeArgs* a, void* stream) {
   if (a->rows <= 0) return 0;
   const int heads_total = a->q_heads + 2 * a->kv_heads;
-  // A CTA per row where the rows alone fill the SMs several times over; in a decode step every head has a warp.
+  // A CTA per row where the rows alone fill the SMs several times over; in a decode step every head has a warp. us, warp a head / CTA a
+  // row, 16 + 8 + 8 heads of 128: 256 rows 3.0 / 3.4, 591 rows 5.2 / 5.6, 1000 rows 8.0 / 6.7; 32 + 8 + 8: 3.9 / 4.5, 7.4 / 7.7,
+  // 11.8 / 9.0.
   const bool many = a->rows >= 148 * 4;
   const dim3 grid(a->rows, many ? 1 : (heads_total + 7) / 8);
   const int step = static_cast<int>(grid.y) * 8;
