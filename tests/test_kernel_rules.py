@@ -66,8 +66,11 @@ def _all_functions():
 
 
 def dependent_kernels(source):
-    return sorted({k for m in re.finditer(r"pdl::launch\(([^,]*),", _plain(source.read_text())) for k in re.findall(r"\b\w+_kernel\b", m.group(1))}
-                  | ({"gemm_ws_kernel"} if source.name == "gemm.cu" else set()))
+    text = _plain(source.read_text())
+    launched = re.findall(r"pdl::launch\(([^,]*),", text)
+    if any(arg.strip() == "kernel" for arg in launched):      # chosen in front of the launch
+        launched += re.findall(r"auto kernel =([^;]*);", text)
+    return sorted({k for arg in launched for k in re.findall(r"\b\w+_kernel\b", arg)})
 
 
 def _reached(source, kernel):

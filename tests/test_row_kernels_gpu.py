@@ -72,3 +72,23 @@ def test_argmax_of_short_rows_back_to_back(vocab):
     torch.cuda.synchronize()
     got = [A.argmax(x) for _ in range(50)]
     assert all(torch.equal(t, want) for t in got)
+
+
+@pytest.mark.parametrize("hidden", [248, 256, 264, 512, 520, 1024, 2040, 2048, 2056, 4096, 4104, 8184])      # pieces a thread holds: 1, 2, 4
+@pytest.mark.parametrize("parts", [1, 2, 4])
+def test_norm_forms_store_the_same_bits(hidden, parts):
+    """Rows of one part, rows of several and rows that a flag guards go through different kernels; sums are in the same order."""
+    from crosspool_b200.ops import norm
+
+    g = torch.Generator(device="cuda").manual_seed(hidden + parts)
+    p = [torch.randn(21, hidden, device="cuda", generator=g).bfloat16() for _ in range(parts)]
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda", generator=g)).bfloat16()
+    r = torch.randn(21, hidden, device="cuda", generator=g).bfloat16()
+    ready = torch.ones(8, device="cuda", dtype=torch.int32)
+    torch.cuda.synchronize()
+    got_r, want_r = r.clone(), r.clone()
+    got = norm.add_rmsnorm(p, w, 1e-6, resid=got_r)
+    want = norm.add_rmsnorm(p, w, 1e-6, resid=want_r, wait_flag_ptrs=[ready.data_ptr()] * parts, wait_seq=1)
+    assert torch.equal(got, want) and torch.equal(got_r, want_r)
+    s = (sum(t.float() for t in p).bfloat16().float() if parts > 1 else p[0].float()) + r.float()
+    assert torch.equal(got_r, s.bfloat16())
