@@ -55,10 +55,13 @@ __device__ __forceinline__ void add8(float (&acc)[8], const uint4& raw) {
 
 // The same arithmetic, in the same order of sums, for rows of one part that neither wait for another GPU nor are sent to one. What bounds it
 // is one round of loads: input, residual and weights of a row are requested together (the weights, where they are the
-// model's, before the previous kernel has ended; in a decode step they come from HBM). kWarp: rows of at most 1024 elements are a
-// warp's, eight rows a CTA, and need no block barrier; wider ones are a CTA's. Beside the general kernel:
-// 6000 rows of 4096 54.4 -> 41.1 us (196 MB: 4.8 TB/s).
-template <bool kWarp>
+// model's, before the previous kernel has ended; in a decode step they come from HBM), and the rows an SM has in flight, so kVec,
+// the 16-byte pieces a thread holds of each, is no more than the row needs. kWarp: rows of at most 1024 elements are a
+// warp's, eight rows a CTA, and need no block barrier; wider ones are a CTA's. us, general kernel / four pieces whatever the row / so:
+// 6000 rows of 1536 20.3 / 22.4 / 11.7, of 2048 23.5 / 24.1 / 13.6, of 4096 52.2 / 39.5 / 31.4 (196 MB: 6.3 TB/s); 1000 rows of 1152
+// 4.9 / 5.1 / 2.9. Rows of several parts stay with the general kernel, which requests one after the other without waiting in between: 16
+// rows of 1024 in 4 parts 2.5 us, a warp per row 5.2.
+template <bool kWarp, int kVec>
 __global__ void __launch_bounds__(kThreads)
 norm_rows_kernel(XpNormArgs a) {
   __shared__ float red[kThreads / 32];
@@ -66,10 +69,10 @@ norm_rows_kernel(XpNormArgs a) {
   const int row = kWarp ? blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5) : blockIdx.x;
   const int first = kWarp ? lane : threadIdx.x, step = kWarp ? 32 : kThreads;
   const int nvec = a.hidden / 8;
-  uint4 w[kMaxVec], x[kMaxVec], r[kMaxVec];
+  uint4 w[kVec], x[kVec], r[kVec];
   auto load_weight = [&] {
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it)
+    for (int it = 0; it < kVec; ++it)
       if (first + it * step < nvec) w[it] = reinterpret_cast<const uint4*>(a.weight)[first + it * step];
   };
   if (a.weight != nullptr && a.w_static) load_weight();
@@ -79,7 +82,7 @@ norm_rows_kernel(XpNormArgs a) {
   const uint4* in = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.parts[0]) + static_cast<size_t>(row) * a.ld_parts);
   uint4* resid = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.resid) + static_cast<size_t>(row) * a.hidden);
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
+  for (int it = 0; it < kVec; ++it) {
     const int v = first + it * step;
     if (v < nvec) {
       x[it] = __ldcg(in + v);
@@ -87,9 +90,9 @@ norm_rows_kernel(XpNormArgs a) {
     }
   }
   if (a.weight != nullptr && !a.w_static) load_weight();
-  float vals[kMaxVec][8], ss[kMaxVec];
+  float vals[kVec][8], ss[kVec];
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
+  for (int it = 0; it < kVec; ++it) {
     ss[it] = 0.f;
     const int v = first + it * step;
     if (v >= nvec) continue;
@@ -117,14 +120,16 @@ norm_rows_kernel(XpNormArgs a) {
   float total;
   if (kWarp) {
     // the sums of the four warps that would share the row in a CTA, added as block_sum adds them
-    static_assert(kMaxVec == 4, "a tree of four");
+    static_assert(kVec == 1 || kVec == 2 || kVec == 4, "a tree of up to four");
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it) ss[it] = warp_sum(ss[it]);
-    total = (ss[0] + ss[2]) + (ss[1] + ss[3]);
+    for (int it = 0; it < kVec; ++it) ss[it] = warp_sum(ss[it]);
+    total = ss[0];
+    if (kVec == 2) total += ss[kVec - 1];
+    if (kVec == 4) total = (ss[0] + ss[kVec / 2]) + (ss[kVec / 4] + ss[kVec - 1]);
   } else {
     float t = 0.f;
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it)
+    for (int it = 0; it < kVec; ++it)
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (first + it * step < nvec) t = fmaf(vals[it][j], vals[it][j], t);
@@ -133,7 +138,7 @@ norm_rows_kernel(XpNormArgs a) {
   const float inv = rsqrtf(total / static_cast<float>(a.hidden) + a.eps);
   uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out_local) + static_cast<size_t>(row) * a.ld_out);
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
+  for (int it = 0; it < kVec; ++it) {
     const int v = first + it * step;
     if (v >= nvec) continue;
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w[it]);
@@ -315,13 +320,14 @@ swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ 
 extern "C" int xp_norm_publish(const XpNormArgs* a, void* stream) {
   if (a->hidden % 8 != 0 || a->hidden > 8 * xpool::norm::kThreads * xpool::norm::kMaxVec) return -10;
   if (a->rows <= 0 || a->nparts < 1 || a->nparts > 8 || a->npeers < 0 || a->npeers > 8) return -11;
-  // Rows of several parts stay with the general kernel, which requests one after the other without waiting in between: 16 rows of
-  // 1024 in 4 parts 2.5 us, a warp per row 5.2.
   if (a->wait_seq == 0 && a->npeers == 0 && a->nparts == 1) {
     using namespace xpool::norm;
     const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    if (a->hidden <= 1024) xpool::pdl::launch(norm_rows_kernel<true>, (a->rows + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, s, 1, *a);
-    else xpool::pdl::launch(norm_rows_kernel<false>, a->rows, kThreads, 0, s, 1, *a);
+    const bool warp = a->hidden <= 1024;
+    const int vec = (a->hidden / 8 + (warp ? 31 : kThreads - 1)) / (warp ? 32 : kThreads);
+    auto kernel = warp ? (vec <= 1 ? norm_rows_kernel<true, 1> : vec <= 2 ? norm_rows_kernel<true, 2> : norm_rows_kernel<true, 4>)
+                       : (vec <= 1 ? norm_rows_kernel<false, 1> : vec <= 2 ? norm_rows_kernel<false, 2> : norm_rows_kernel<false, 4>);
+    xpool::pdl::launch(kernel, warp ? (a->rows + kThreads / 32 - 1) / (kThreads / 32) : a->rows, kThreads, 0, s, 1, *a);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
   }
