@@ -30,9 +30,9 @@ __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// Greedy sampling. A cluster of eight CTAs takes a row, 16 bytes a load (one 1024-thread CTA with 2-byte loads took 13.5 us for 152k
-// bf16 logits, bound by the latency of a thread's 150 loads in a row); the eight winners meet in the first CTA's shared memory.
-constexpr int kArgCluster = 8, kArgThreads = 256;
+// Greedy sampling. A cluster of up to eight CTAs takes a row, 16 bytes a load (one 1024-thread CTA with 2-byte loads took 13.5 us for 152k
+// bf16 logits, bound by the latency of a thread's 150 loads in a row); the winners meet in the first CTA's shared memory.
+constexpr int kArgCluster = 8;
 
 __device__ __forceinline__ void better(float& best, int& bi, float v, int i) {
   if (v > best || (v == best && i < bi)) best = v, bi = i;
@@ -46,32 +46,31 @@ __device__ __forceinline__ void warp_best(float& best, int& bi) {
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kArgThreads)
-argmax_kernel(const T* logits, int* out, int vocab, int ld, int wide) {
+template <typename T, int kThreads>
+__global__ void __launch_bounds__(kThreads)
+argmax_kernel(const T* logits, int* out, int vocab, int ld, int wide, int ranks) {
   namespace cg = cooperative_groups;
   // The first CTA's shared memory may be written once that CTA is known to have started: all arrive here and wait before the
   // stores, a row's scan later.
   auto started = cg::this_cluster().barrier_arrive();
   xpool::pdl::wait();
   xpool::pdl::release();
-  constexpr int N = 16 / sizeof(T), kWarps = kArgThreads / 32;
-  __shared__ float sv[kArgCluster * kWarps];
-  __shared__ int si[kArgCluster * kWarps];
-  const int rank = blockIdx.x % kArgCluster, at = blockIdx.x / kArgCluster, first = rank * kArgThreads + threadIdx.x;
-  constexpr int kStride = kArgCluster * kArgThreads;
+  constexpr int N = 16 / sizeof(T), kWarps = kThreads / 32, kSlots = kThreads == 256 ? kArgCluster * kWarps : kWarps;
+  __shared__ float sv[kSlots];
+  __shared__ int si[kSlots];
+  const int rank = blockIdx.x % ranks, at = blockIdx.x / ranks, first = rank * kThreads + threadIdx.x, stride = ranks * kThreads;
   const T* row = logits + static_cast<size_t>(at) * ld;
   float best = -CUDART_INF_F;
   int bi = 0x7fffffff;
   const int whole = wide ? vocab / N : 0;
 #pragma unroll 4
-  for (int c = first; c < whole; c += kStride) {
+  for (int c = first; c < whole; c += stride) {
     const uint4 raw = reinterpret_cast<const uint4*>(row)[c];
     const T* v = reinterpret_cast<const T*>(&raw);
 #pragma unroll
     for (int j = 0; j < N; ++j) better(best, bi, to_f<T>(v[j]), c * N + j);
   }
-  for (int i = whole * N + first; i < vocab; i += kStride) better(best, bi, to_f<T>(row[i]), i);
+  for (int i = whole * N + first; i < vocab; i += stride) better(best, bi, to_f<T>(row[i]), i);
   warp_best(best, bi);
   cg::this_cluster().barrier_wait(std::move(started));
   if ((threadIdx.x & 31) == 0) {
@@ -82,7 +81,7 @@ argmax_kernel(const T* logits, int* out, int vocab, int ld, int wide) {
   cg::this_cluster().sync();
   if (rank != 0 || threadIdx.x >= 32) return;
   best = -CUDART_INF_F, bi = 0x7fffffff;
-  for (int i = threadIdx.x; i < kArgCluster * kWarps; i += 32) better(best, bi, sv[i], si[i]);
+  for (int i = threadIdx.x; i < ranks * kWarps; i += 32) better(best, bi, sv[i], si[i]);
   warp_best(best, bi);
   if (threadIdx.x == 0) out[at] = bi;
 }
@@ -183,12 +182,21 @@ extern "C" int xp_argmax(const void* logits, int is_fp32, int* out, int rows, in
   if (rows <= 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int wide = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && static_cast<size_t>(ld) * (is_fp32 ? 4 : 2) % 16 == 0;
-  const dim3 grid(static_cast<unsigned>(rows) * kArgCluster);
-  if (is_fp32)
-    xpool::pdl::launch(argmax_kernel<float>, grid, kArgThreads, 0, s, kArgCluster, reinterpret_cast<const float*>(logits), out, vocab, ld, wide);
-  else
-    xpool::pdl::launch(argmax_kernel<__nv_bfloat16>, grid, kArgThreads, 0, s, kArgCluster, reinterpret_cast<const __nv_bfloat16*>(logits), out,
-                       vocab, ld, wide);
+  // Clusters while the rows leave SMs idle and every CTA has 4 KB of its row; otherwise a CTA a row, of more threads the longer it is. us,
+  // clusters of eight / so: 8 rows of 151936 bf16 3.7 both; 64 rows 6.5 / 6.1; 256 rows 16.9 / 15.4; 256 rows of 32000 8.8 / 4.9, of 1000
+  // 6.0 / 2.1 (one scalar 1024-thread CTA a row: 11.7, 12.0, 20.9, 6.8, 2.6).
+  const size_t bytes = static_cast<size_t>(vocab) * (is_fp32 ? 4 : 2);
+  int ranks = rows <= 32 ? 8 : rows <= 64 ? 4 : 1;
+  while (ranks > 1 && bytes / ranks < 4096) ranks >>= 1;
+  const int threads = ranks > 1 || bytes <= 8192 ? 256 : bytes <= 65536 ? 512 : 1024;
+  auto go = [&](auto kernel, auto* p) { xpool::pdl::launch(kernel, static_cast<unsigned>(rows) * ranks, threads, 0, s, ranks, p, out, vocab, ld, wide, ranks); };
+  if (is_fp32) {
+    const float* p = reinterpret_cast<const float*>(logits);
+    go(threads == 256 ? argmax_kernel<float, 256> : threads == 512 ? argmax_kernel<float, 512> : argmax_kernel<float, 1024>, p);
+  } else {
+    const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(logits);
+    go(threads == 256 ? argmax_kernel<__nv_bfloat16, 256> : threads == 512 ? argmax_kernel<__nv_bfloat16, 512> : argmax_kernel<__nv_bfloat16, 1024>, p);
+  }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }

@@ -68,8 +68,9 @@ def _all_functions():
 def dependent_kernels(source):
     text = _plain(source.read_text())
     launched = re.findall(r"pdl::launch\(([^,]*),", text)
-    if any(arg.strip() == "kernel" for arg in launched):      # chosen in front of the launch
-        launched += re.findall(r"auto kernel =([^;]*);", text)
+    if any(arg.strip() == "kernel" for arg in launched):      # chosen in front of the launch, or handed to a lambda that launches it
+        launched += re.findall(r"auto kernel =([^;]*);|\bgo\(([^;]*), p\);", text)
+        launched = ["".join(arg) for arg in launched]
     return sorted({k for arg in launched for k in re.findall(r"\b\w+_kernel\b", arg)})
 
 

@@ -92,3 +92,18 @@ def test_norm_forms_store_the_same_bits(hidden, parts):
     assert torch.equal(got, want) and torch.equal(got_r, want_r)
     s = (sum(t.float() for t in p).bfloat16().float() if parts > 1 else p[0].float()) + r.float()
     assert torch.equal(got_r, s.bfloat16())
+
+
+# a cluster of 8, 4 or 2 CTAs a row, a CTA of 256, 512 or 1024 threads; the winner in any of their parts, ties between parts
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows", [1, 32, 33, 64, 65, 300])
+@pytest.mark.parametrize("vocab", [1000, 4096, 8200, 20000, 32768, 33001])
+def test_argmax_forms(vocab, rows, dtype):
+    from crosspool_b200.ops import attention as A
+
+    g = torch.Generator(device="cuda").manual_seed(vocab + rows)
+    x = torch.rand(rows, vocab, device="cuda", generator=g).to(dtype)
+    at = torch.randint(0, vocab, (rows,), device="cuda", generator=g)
+    x[torch.arange(rows, device="cuda"), at] = 2
+    x[torch.arange(rows, device="cuda"), (at + vocab // 3) % vocab] = 2
+    assert torch.equal(A.argmax(x), torch.minimum(at, (at + vocab // 3) % vocab).int())
