@@ -52,18 +52,34 @@ __device__ __forceinline__ void tile_f32(const float* __restrict__ x, const floa
   const int slices = (k + kBK - 1) / kBK;
   auto load = [&](int slice, int stage) {
     const int k0 = slice * kBK;
-    constexpr int kUnit = VEC ? 4 : 1, kUnits = kBK / kUnit;
+    if constexpr (VEC) {
+      constexpr int kUnits = kBK / 4;
 #pragma unroll 8
-    for (int i = t; i < (kBM + kBN) * kUnits; i += kGroup) {
-      const int m = i / kUnits, c = k0 + i % kUnits * kUnit;
-      const bool of_x = m < kBM;
-      const int row = of_x ? r0 + m : n0 + m - kBM;
-      const bool in = row < (of_x ? rows : n) && c < k;
-      const float* src = of_x ? x : w;
-      if (in) src += static_cast<int64_t>(row) * (of_x ? ldx : ldw) + c;
-      const uint32_t dst = base + (stage * kStage + m * kPitch + i % kUnits * kUnit) * 4;
-      if constexpr (VEC) copy16(dst, src, in ? min(4, k - c) * 4 : 0);
-      else copy4(dst, src, in ? 4 : 0);
+      for (int i = t; i < (kBM + kBN) * kUnits; i += kGroup) {
+        const int m = i / kUnits, c = k0 + i % kUnits * 4;
+        const bool of_x = m < kBM;
+        const int row = of_x ? r0 + m : n0 + m - kBM;
+        const bool in = row < (of_x ? rows : n) && c < k;
+        const float* src = of_x ? x : w;
+        if (in) src += static_cast<int64_t>(row) * (of_x ? ldx : ldw) + c;
+        copy16(base + (stage * kStage + m * kPitch + i % kUnits * 4) * 4, src, in ? min(4, k - c) * 4 : 0);
+      }
+    } else {
+      // an element a copy, so the instructions around it count: a thread keeps its column and steps from row to row of one operand
+      // (2048 rows x 1001 features x 999: 209 us with both operands' rows worked out for every copy)
+      static_assert(kBK == 32 && kGroup % 32 == 0, "a warp copies a row's slice");
+      constexpr int kStep = kGroup / 32;
+      const int c = k0 + (t & 31), m0 = t >> 5;
+      auto rows_of = [&](const float* src, int ld, int first, int end, int count, int at) {
+        const float* p = src + static_cast<int64_t>(first + m0) * ld + c;
+        uint32_t dst = base + (stage * kStage + (at + m0) * kPitch + (t & 31)) * 4;
+        int left = c < k ? end - first - m0 : 0;
+#pragma unroll 8
+        for (int j = 0; j < count / kStep; ++j, left -= kStep, p += static_cast<int64_t>(kStep) * ld, dst += kStep * kPitch * 4)
+          copy4(dst, left > 0 ? p : src, left > 0 ? 4 : 0);
+      };
+      rows_of(x, ldx, r0, rows, kBM, 0);
+      rows_of(w, ldw, n0, n, kBN, kBM);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
