@@ -212,21 +212,31 @@ gemm_stream_kernel(const __grid_constant__ StreamArgs a) {
   cg::this_cluster().sync();     // nobody's shared memory goes while another CTA reads it
 }
 
-// Rows: the tiled kernel has a fixed cost of 8 us a launch, this one reads the activations once per CTA from L2 and once per warp
-// through L1. us a launch, inputs colder than L2, tiled -> this kernel:
-//                          1 row           8 rows          16 rows         32 rows (four eights a warp)
-//   4096 x 1024            9.3 -> 3.1      9.4 -> 3.3      9.5 -> 4.1      10.8 -> 6.8
-//   gate/up 6144 x 1024    10.9 -> 3.6     10.9 -> 3.8     11.0 -> 4.7     11.7 -> 7.9
-//   1024 x 3072            10.7 -> 4.0     10.7 -> 4.4     10.8 -> 5.0     10.5 -> 8.5
-//   151936 x 1024          73.1 -> 52.5    73.3 -> 59.3    73.9 -> 69.5    75.5 -> 117
-//   gate/up 24576 x 4096   42.5 -> 36.7    42.2 -> 38.1    42.1 -> 41.8    41.4 -> 73.6
-//   4096 x 12288           29.7 -> 17.8    29.6 -> 18.4    29.7 -> 20.7    31.1 -> 33.8
+// Rows: the tiled kernel has a fixed cost of 6 us a launch, this one reads the activations once per CTA from L2 and once per warp
+// through L1. us a launch, inputs colder than L2, tiled / this kernel:
+//                          1 row           8 rows          16 rows
+//   4096 x 1024            6.8 / 3.2       6.8 / 3.3       6.8 / 4.2
+//   gate/up 6144 x 1024    8.2 / 3.8       8.2 / 3.9       8.2 / 4.8
+//   1024 x 3072            8.3 / 4.1       8.3 / 4.4       8.3 / 5.1
+//   6144 x 4096            12.6 / 10.7     12.6 / 11.2     12.6 / 11.5
+//   gate/up 16384 x 2560   17.5 / 14.4     17.4 / 14.7     17.5 / 15.8
+//   4096 x 12288           21.5 / 16.8     21.6 / 17.5     21.7 / 19.6
+//   3584 x 18944           27.2 / 23.2     27.3 / 24.3     27.2 / 28.0
+//   gate/up 24576 x 4096   36.1 / 36.7     36.2 / 37.3     36.2 / 40.9
+//   gate/up 37888 x 3584   41.3 / 47.3     41.5 / 48.1     41.6 / 49.0
+//   151936 x 1024          51.9 / 49.3     52.5 / 55.6     53.0 / 66.7    (4 rows: 52.4 / 52.1)
+//   151936 x 4096          194 / 189       196 / 199       198 / 206      (4 rows: 194 / 195)
+// (a form with four eights a warp lost at 32 rows: 24576 x 4096 73.6 us.) So matrices of more than kStreamManyBytes, whose reading hides
+// the tiled kernel's fixed cost, come here with up to four rows, gated ones not at all.
 // From two eights on a warp takes 32 features, which halves what it reads of the activations. Calls that name a tile width,
 // a split or an SM count mean the tiled kernel; rows of K that are no whole 16-byte units, and features whose weight rows the caller
 // says do not exist (w_rows_total), need its zero-filled tiles.
+constexpr int64_t kStreamManyBytes = 150 << 20;
+
 bool stream_applies(const XpGemmArgs& a) {
   const int groups = a.batch > 1 ? a.batch - 1 : 0;
   const int64_t w_rows = a.n_out + static_cast<int64_t>(groups) * a.w_rows_per_group + (a.dual ? a.up_offset : 0);
+  if (w_rows * a.k * 2 > kStreamManyBytes && (a.dual || a.rows > 4)) return false;
   if (a.w_rows_total > 0 && (a.w_rows_total < w_rows || (a.w_tiled && a.w_rows_total % kTileM != 0))) return false;
   const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return a.rows <= kStreamMaxRows && !a.fp8 && a.tile_table == nullptr && a.splits == 0 && a.bn == 0 && a.num_sms == 0 && a.k % 8 == 0 &&
@@ -240,7 +250,7 @@ static int stream_go(const StreamArgs& s, dim3 grid, cudaStream_t stream) {
   return e == cudaSuccess ? 0 : -100 - static_cast<int>(e);
 }
 
-// How K is cut: estimated time (us) of a launch by waves of CTAs (two per SM), each at its share of 6.4 TB/s and at most 40 GB/ms,
+// How K is cut: estimated time (us) of a launch by waves of CTAs (two per SM), each at its share of 6.4 TB/s and at most 40 GB/s,
 // plus a fixed microsecond a wave and another for the cluster's two barriers. Only the order of the estimates matters.
 static void stream_split(StreamArgs* s, int n_out, int batch, int k, int dual, int feats) {
   const int steps = (k + kSStep - 1) / kSStep;

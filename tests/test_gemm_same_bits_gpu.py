@@ -82,3 +82,12 @@ def test_batched_products(rows):
     gate = r.view(rows, -1)[:, :heads * n].contiguous()
     _same(x, w, n, rows, batch=heads, epilogue=gemm.EPI_STORE)
     _same(x, w, n, rows, batch=heads, epilogue=gemm.EPI_SIGMOID, resid=gate)
+
+
+@pytest.mark.parametrize("rows,n,k,dual", [(4, 19204, 4096, 0), (5, 19204, 4096, 0), (4, 19200, 4096, 0), (16, 19200, 4096, 0), (1, 9601, 4096, 1), (1, 9600, 4096, 1)])
+def test_large_matrices_at_the_limits_of_the_streamed_form(rows, n, k, dual):
+    """150 MB of weights, four rows, gated or not: either side of each line gives the tiled form's bits."""
+    from crosspool_b200.ops import gemm
+
+    x, w, _, _ = _operands(rows, n * (2 if dual else 1), k, rows + n)
+    _same(x, w, n, rows, **(dict(epilogue=gemm.EPI_SWIGLU, dual=1, up_offset=n) if dual else dict(epilogue=gemm.EPI_STORE)))
