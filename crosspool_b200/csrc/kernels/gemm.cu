@@ -71,8 +71,9 @@ __device__ __forceinline__ void run_tiles(const Problem& p, int nacc, int smem_b
 }
 
 // At most 208 registers: 192 threads x 208 leave room on the SM for one decode-attention CTA of another
-// stream (128 threads x 192 registers), which is how decode GEMMs hide behind the co-located Instance's
-// attention.
+// stream (128 threads x 192 registers), which is how decode products of more than 16 rows hide behind the
+// co-located Instance's attention. (Those of up to 16 rows, gemm_stream.cu, fill the register file and leave it
+// in half the time.)
 template <bool kWide>
 __global__ void __maxnreg__(208)
 gemm_ws_kernel(const __grid_constant__ CUtensorMap tmap_w,

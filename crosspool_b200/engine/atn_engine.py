@@ -107,7 +107,9 @@ class UnsupportedAttention(NotImplementedError):
 
 class FfnPort:
     """Where a layer's FFN runs. ``run`` receives the normalised hidden states of ``rows`` tokens
-    and returns the tensors whose fixed-order sum is the FFN output (one per FFN TP rank)."""
+    and returns the tensors whose fixed-order sum is the FFN output (one per FFN TP rank). It is called inside a
+    forward pass: the kernel before it on the stream wrote ``x``, so ports may begin to read their weights before
+    that kernel has ended."""
 
     def attach(self, engine: "AttentionEngine") -> None:  # pragma: no cover - interface
         pass
